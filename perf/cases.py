@@ -56,7 +56,7 @@ def listed():
         # LES at 128^3, Re 6000: Smagorinsky; the dynamic localization model (a transported k_sgs); the learned closure
         _dns("les_128_smagorinsky", 128, 50, les=1, re=6000.0, spectrum=3),
         _dns("les_128_dynamic", 128, 30, les=2, re=6000.0, spectrum=3),
-        _dns("les_128_learned", 128, 4, les=20, re=6000.0, spectrum=3),
+        _dns("les_128_learned", 128, 50, les=20, re=6000.0, spectrum=3),
         # the statistics a run takes every IPRINT1 steps: velocity and two scalars at 256^3
         dict(name="stats_256", kind="stats", n=256, scalars=2, re=1000.0),
         # a host that owns its fields: 2/3-rule band up, one step, band down, eight states in flight
@@ -85,7 +85,7 @@ def draw(rng):
     if kind == "les":
         n = rng.choice([32, 48, 64, 128])
         les = rng.choice([1, 1, 2, 20, 20])
-        c = _dns("", n, rng.randrange(2, 6) if les == 20 else rng.randrange(5, 40), les=les, re=re, dt=0.128 / n, spectrum=3,
+        c = _dns("", n, rng.randrange(5, 40), les=les, re=re, dt=0.128 / n, spectrum=3,
                  precision=rng.randrange(2) if les == 1 else 0)
     else:
         n = rng.choice([32, 48, 64, 128, 256])
