@@ -570,53 +570,133 @@ __global__ void k_count_nonfinite(int n, int nh, int pitch, int64_t fs, int nf, 
 }
 
 // Shell spectrum sum_{shell} fac * |f|^2 (kx = 0 halved, kx = N/2 excluded),
-// float32 shell index (m_stats.f90:195-235).  Deterministic: each warp owns a
-// private histogram, lane L accumulates the shells congruent to L mod 32 in a
-// fixed element order; warps and blocks are combined in index order.
+// float32 shell index (m_stats.f90:195-235), and, by MODE, the sum of |F|^2 of
+// the vorticity of (u, v, w) (SPEC_CURL) or of the gradient of one field
+// (SPEC_GRAD) over all modes of the real field, which is N^6 times the mean
+// square in physical space (Parseval), so that neither needs a transform.
+//
+// A warp takes 32 adjacent kx of one (ky, kz) row at a time.  |k| grows along
+// the row, so equal shells are adjacent lanes: five shuffle steps sum each run
+// of equal shells and its last lane adds it to the warp's histogram.  (Handing
+// every lane's value to a lane that owns its shell took 32 steps of three
+// shuffles and left the pass bound by them: 256^3 velocity 0.39 ms, now 0.052
+// with the enstrophy's sum in it, 0.4 GB at the kept modes.)
+// Each warp's histogram, then warps, then blocks are added in index order:
+// deterministic.
 // w0 is the weight of the kx = 0 plane: 0.5 for the statistics (m_stats.f90:222),
-// 1 for the decaying-run rescale (velocity_rescale.f90:47-55)
-__global__ void k_shell_partial(int n, int nh, int pitch, int64_t fs, int nf, int kmax, double w0,
-                                const double2 *__restrict__ U, double *__restrict__ part /* [gridDim.x][kmax] */)
+// 1 for the decaying-run rescale (velocity_rescale.f90:47-55).
+// kc >= 0: the state is zero beyond |k_i| = kc, only those modes are read.
+enum SpecMode : int { SPEC_ONLY = 0, SPEC_CURL = 1, SPEC_GRAD = 2 };
+
+// k x u (SPEC_CURL, three components) or k phi (SPEC_GRAD) of one mode; the
+// derivative is i times it
+template <int MODE> H3D_D void spec_deriv(double kx, double ky, double kz, const double2 *v, double2 (&g)[3])
+{
+    if constexpr (MODE == SPEC_CURL) {
+        g[0] = make_double2(ky * v[2].x - kz * v[1].x, ky * v[2].y - kz * v[1].y);
+        g[1] = make_double2(kz * v[0].x - kx * v[2].x, kz * v[0].y - kx * v[2].y);
+        g[2] = make_double2(kx * v[1].x - ky * v[0].x, kx * v[1].y - ky * v[0].y);
+    } else {
+        g[0] = make_double2(kx * v[0].x, kx * v[0].y);
+        g[1] = make_double2(ky * v[0].x, ky * v[0].y);
+        g[2] = make_double2(kz * v[0].x, kz * v[0].y);
+    }
+}
+
+template <int MODE, int NF>
+__global__ void __launch_bounds__(256) k_shell_partial(int n, int pitch, int64_t fs, int kmax, double w0, int kc,
+                                                       const double2 *__restrict__ U,
+                                                       double *__restrict__ part /* [gridDim.x][kmax] */,
+                                                       double *__restrict__ psum /* [gridDim.x] */)
 {
     extern __shared__ double hist[];  // [warps][kmax]
+    __shared__ double wsum[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int i = threadIdx.x; i < nw * kmax; i += blockDim.x) hist[i] = 0.0;
     __syncthreads();
     const double n3 = (double)n * n * n;
     const double fac = 1.0 / (n3 * n3);
-    const int64_t nm = (int64_t)n * n * nh;
-    const int64_t per_block = (nm + gridDim.x - 1) / gridDim.x;
-    const int64_t b0 = blockIdx.x * per_block, b1 = min(nm, b0 + per_block);
+    const int nx = kc >= 0 ? kc + 1 : n / 2;  // kx = N/2 carries no shell
+    const int nr = kc >= 0 ? 2 * kc + 1 : n;
+    const int nch = (nx + 31) / 32;
+    auto axis = [&](int y) { return kc >= 0 && y > kc ? n - (nr - y) : y; };  // kept index -> storage index
     double *h = hist + warp * kmax;
-    for (int64_t base = b0 + warp * 32; base < b1; base += nw * 32) {
-        int64_t t = base + lane;
-        int sh = -1;
+    double ps = 0.0;
+    const unsigned total = (unsigned)nr * nr * nch;  // at most 2^24
+#pragma unroll 2
+    for (unsigned q = blockIdx.x * nw + warp; q < total; q += gridDim.x * nw) {
+        const unsigned r = q / (unsigned)nch, ch = q - r * (unsigned)nch;
+        const int kzi = axis((int)(r / (unsigned)nr)), kyi = axis((int)(r % (unsigned)nr));
+        const int kx = (int)ch * 32 + lane;
+        const double ky = kwave(kyi, n), kz = kwave(kzi, n);
+        int sh = 0x7fffffff;
         double e = 0.0;
-        if (t < b1) {
-            ModeIdx m = mode_of(t, n, nh);
-            if (m.kx < n / 2) {
-                double k2 = m.ax * m.ax + m.ay * m.ay + m.az * m.az;
-                int s = shell32(k2);
-                if (s > 0 && s <= kmax) {
-                    int64_t o = soff(m, n, pitch);
-                    double re = 0.0, im = 0.0;
-                    for (int f = 0; f < nf; f++) {
-                        double2 v = U[o + f * fs];
-                        re = (f == 0) ? v.x * v.x : re + v.x * v.x;
-                        im = (f == 0) ? v.y * v.y : im + v.y * v.y;
-                    }
-                    double e1 = fac * re, e2 = fac * im;
-                    if (m.kx == 0) { e1 *= w0; e2 *= w0; }
-                    e = e1 + e2;
-                    sh = s - 1;
+        if (kx < nx) {
+            const int64_t o = ((int64_t)kzi * n + kyi) * pitch + kx;
+            double2 v[NF];
+#pragma unroll
+            for (int f = 0; f < NF; f++) v[f] = U[o + f * fs];
+            double re = v[0].x * v[0].x, im = v[0].y * v[0].y;
+#pragma unroll
+            for (int f = 1; f < NF; f++) {
+                re = re + v[f].x * v[f].x;
+                im = im + v[f].y * v[f].y;
+            }
+            double e1 = fac * re, e2 = fac * im;
+            if (kx == 0) { e1 *= w0; e2 *= w0; }
+            e = e1 + e2;
+            sh = shell32((double)kx * kx + ky * ky + kz * kz);
+            if constexpr (MODE != SPEC_ONLY) {
+                if (kx > 0) {  // with the conjugate mode at -kx; kx = 0 below
+                    double2 g[3];
+                    spec_deriv<MODE>((double)kx, ky, kz, v, g);
+                    double t = 0.0;
+#pragma unroll
+                    for (int d = 0; d < 3; d++) t = t + (g[d].x * g[d].x + g[d].y * g[d].y);
+                    ps += 2.0 * t;
                 }
             }
         }
-        for (int l = 0; l < 32; l++) {
-            int s = __shfl_sync(0xffffffffu, sh, l);
-            double v = __shfl_sync(0xffffffffu, e, l);
-            if (s >= 0 && (s & 31) == lane) h[s] += v;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const double ev = __shfl_up_sync(0xffffffffu, e, off);
+            const int sv = __shfl_up_sync(0xffffffffu, sh, off);
+            if (lane >= off && sv == sh) e += ev;
         }
+        const int next = __shfl_down_sync(0xffffffffu, sh, 1);
+        if (sh > 0 && sh <= kmax && (lane == 31 || next != sh)) h[sh - 1] += e;
+        __syncwarp();
+    }
+    if constexpr (MODE != SPEC_ONLY) {
+        // the planes kx = 0 and N/2, where the x transform keeps the part of the
+        // field that is conjugate to its mirror mode
+        const int np = kc >= 0 ? 1 : 2;
+        const int64_t nm = (int64_t)np * nr * nr;
+        for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nm; t += (int64_t)gridDim.x * blockDim.x) {
+            const unsigned r = (unsigned)(t / np);
+            const int kx = (t % np) ? n / 2 : 0;
+            const int kzi = axis((int)(r / (unsigned)nr)), kyi = axis((int)(r % (unsigned)nr));
+            const int mz = kzi ? n - kzi : 0, my = kyi ? n - kyi : 0;
+            const int64_t o = ((int64_t)kzi * n + kyi) * pitch + kx, om = ((int64_t)mz * n + my) * pitch + kx;
+            double2 v[NF], w[NF], g[3], gm[3];
+#pragma unroll
+            for (int f = 0; f < NF; f++) {
+                v[f] = U[o + f * fs];
+                w[f] = U[om + f * fs];
+            }
+            // the mirror of kx = N/2 is stored as +N/2 again, its x wavenumber too
+            spec_deriv<MODE>((double)kx, kwave(kyi, n), kwave(kzi, n), v, g);
+            spec_deriv<MODE>((double)kx, kwave(my, n), kwave(mz, n), w, gm);
+            double s = 0.0;
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const double a = 0.5 * (g[d].x - gm[d].x), b = 0.5 * (g[d].y + gm[d].y);
+                s = s + (a * a + b * b);
+            }
+            ps += s;
+        }
+        for (int off = 16; off > 0; off >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, off);
+        if (lane == 0) wsum[warp] = ps;
     }
     __syncthreads();
     for (int s = threadIdx.x; s < kmax; s += blockDim.x) {
@@ -624,42 +704,65 @@ __global__ void k_shell_partial(int n, int nh, int pitch, int64_t fs, int nf, in
         for (int w = 0; w < nw; w++) acc += hist[w * kmax + s];
         part[(int64_t)blockIdx.x * kmax + s] = acc;
     }
+    if (MODE != SPEC_ONLY && threadIdx.x == 0) {
+        double acc = 0.0;
+        for (int w = 0; w < nw; w++) acc += wsum[w];
+        psum[blockIdx.x] = acc;
+    }
 }
 
-__global__ void k_shell_final(int nblk, int kmax, const double *__restrict__ part, double *__restrict__ out)
+// shells s < kmax, and the Parseval sum (psum != nullptr) as entry kmax: one warp
+// each, the blocks strided over its lanes, then a fixed shuffle tree (one thread
+// walking the blocks took a chain of nblk loads)
+__global__ void k_shell_final(int nblk, int kmax, const double *__restrict__ part, const double *__restrict__ psum,
+                              double *__restrict__ out)
 {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < kmax; s += gridDim.x * blockDim.x) {
-        double acc = 0.0;
-        for (int b = 0; b < nblk; b++) acc += part[(int64_t)b * kmax + s];
-        out[s] = acc;
-    }
+    const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (s > kmax || (s == kmax && psum == nullptr)) return;
+    const double *p = s < kmax ? part + s : psum;
+    const int64_t st = s < kmax ? kmax : 1;
+    double acc = 0.0;
+    for (int b = lane; b < nblk; b += 32) acc += p[b * st];
+    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (lane == 0) out[s] = acc;
 }
 
 // Deterministic sums over physical points of the fields:
 // mode 0: sum_f x_f^2;  mode 1: x_0^2 and x_0^3 (two sums);  mode 2: x, x^2, min, max of x_0
-__global__ void k_phys_partial(int n, int64_t rpitch, int64_t fs, int nf, int mode, const double *__restrict__ X,
-                               double *__restrict__ part /* [gridDim.x][4] */)
+// of the field (or first of nf fields) at X + blockIdx.y fs.  A warp walks whole
+// rows, 16 bytes a lane (rows start on 16 bytes: the pitch is even), with no
+// division per point: one field of 256^3 takes 0.024 ms (134 MB), where a 64-bit
+// division per point took 0.15.
+__global__ void __launch_bounds__(256) k_phys_partial(int n, int64_t rpitch, int64_t fs, int nf, int mode,
+                                                      const double *__restrict__ X,
+                                                      double *__restrict__ part /* [gridDim.y][gridDim.x][4] */)
 {
-    __shared__ double sh[4][32];
-    const int64_t np = (int64_t)n * n * n;
+    __shared__ double sh[4][8];
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int rows = n * n, nv = n / 2;
+    X += blockIdx.y * fs;
     double s0 = 0.0, s1 = 0.0, mn = 1e300, mx = -1e300;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < np; t += (int64_t)gridDim.x * blockDim.x) {
-        int64_t row = t / n, x = t - row * n;
-        const double *p = X + row * rpitch + x;
-        if (mode == 0) {
-            double q = 0.0;
-            for (int f = 0; f < nf; f++) { double v = p[f * fs]; q = (f == 0) ? v * v : q + v * v; }
-            s0 += q;
-        } else if (mode == 1) {
-            double v = p[0];
-            s0 += v * v;
-            s1 += v * v * v;
-        } else {
-            double v = p[0];
-            s0 += v;
-            s1 += v * v;
-            mn = fmin(mn, v);
-            mx = fmax(mx, v);
+    for (int row = blockIdx.x * nw + w; row < rows; row += gridDim.x * nw) {
+        const double *p = X + row * rpitch;
+#pragma unroll 4
+        for (int x = l; x < nv; x += 32) {
+            const double2 v = reinterpret_cast<const double2 *>(p)[x];
+            if (mode == 0) {
+                double2 q = make_double2(v.x * v.x, v.y * v.y);
+                for (int f = 1; f < nf; f++) {
+                    const double2 u = reinterpret_cast<const double2 *>(p + f * fs)[x];
+                    q = make_double2(q.x + u.x * u.x, q.y + u.y * u.y);
+                }
+                s0 += q.x + q.y;
+            } else if (mode == 1) {
+                s0 += v.x * v.x + v.y * v.y;
+                s1 += v.x * v.x * v.x + v.y * v.y * v.y;
+            } else {
+                s0 += v.x + v.y;
+                s1 += v.x * v.x + v.y * v.y;
+                mn = fmin(mn, fmin(v.x, v.y));
+                mx = fmax(mx, fmax(v.x, v.y));
+            }
         }
     }
     for (int off = 16; off > 0; off >>= 1) {
@@ -668,26 +771,36 @@ __global__ void k_phys_partial(int n, int64_t rpitch, int64_t fs, int nf, int mo
         mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, off));
         mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     }
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
     if (l == 0) { sh[0][w] = s0; sh[1][w] = s1; sh[2][w] = mn; sh[3][w] = mx; }
     __syncthreads();
     if (threadIdx.x == 0) {
         double a0 = 0.0, a1 = 0.0, a2 = 1e300, a3 = -1e300;
         for (int i = 0; i < nw; i++) { a0 += sh[0][i]; a1 += sh[1][i]; a2 = fmin(a2, sh[2][i]); a3 = fmax(a3, sh[3][i]); }
-        part[blockIdx.x * 4 + 0] = a0; part[blockIdx.x * 4 + 1] = a1;
-        part[blockIdx.x * 4 + 2] = a2; part[blockIdx.x * 4 + 3] = a3;
+        double *o = part + 4 * ((int64_t)blockIdx.y * gridDim.x + blockIdx.x);
+        o[0] = a0; o[1] = a1; o[2] = a2; o[3] = a3;
     }
 }
 
+// one warp per field (blockIdx.x): the blocks strided over its lanes, then a
+// fixed shuffle tree
 __global__ void k_phys_final(int nblk, const double *__restrict__ part, double *__restrict__ out)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    const double *p = part + 4 * (int64_t)blockIdx.x * nblk;
     double a0 = 0.0, a1 = 0.0, a2 = 1e300, a3 = -1e300;
-    for (int b = 0; b < nblk; b++) {
-        a0 += part[b * 4]; a1 += part[b * 4 + 1];
-        a2 = fmin(a2, part[b * 4 + 2]); a3 = fmax(a3, part[b * 4 + 3]);
+    for (int b = threadIdx.x; b < nblk; b += 32) {
+        a0 += p[b * 4]; a1 += p[b * 4 + 1];
+        a2 = fmin(a2, p[b * 4 + 2]); a3 = fmax(a3, p[b * 4 + 3]);
     }
-    out[0] = a0; out[1] = a1; out[2] = a2; out[3] = a3;
+    for (int off = 16; off > 0; off >>= 1) {
+        a0 += __shfl_xor_sync(0xffffffffu, a0, off);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, off);
+        a2 = fmin(a2, __shfl_xor_sync(0xffffffffu, a2, off));
+        a3 = fmax(a3, __shfl_xor_sync(0xffffffffu, a3, off));
+    }
+    if (threadIdx.x == 0) {
+        double *o = out + 4 * blockIdx.x;
+        o[0] = a0; o[1] = a1; o[2] = a2; o[3] = a3;
+    }
 }
 
 // ---------------------------------------------------------------------------
