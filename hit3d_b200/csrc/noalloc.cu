@@ -20,10 +20,10 @@
 //   * all calls share the one array: calls whose work overlaps on the GPU (on
 //     different streams, or from different threads) race on it and must be
 //     serialised by the caller.  Nothing in the array needs to start at zero:
-//     each call first copies its whole input into it;
-//   * input and output may be the same buffer, or overlap: the whole input is
-//     copied into the array, in stream order, before anything is written to the
-//     output.
+//     each call first fills it;
+//   * input and output may be the same buffer, or overlap: the x and y
+//     transforms of the whole input reach the array, in stream order, before
+//     anything is written to the output.
 #include <cmath>
 #include <mutex>
 #include <vector>
@@ -89,6 +89,8 @@ int tw_offset(int n)
     return n == 32 ? kTwOff32 : n == 48 ? kTwOff48 : n == 64 ? kTwOff64 : kTwOff128;
 }
 
+int plane_attrs();  // shared-memory limits of the plane kernels
+
 // once per device and CUDA context, with that device current
 int setup_device(int dev)
 {
@@ -118,9 +120,78 @@ int setup_device(int dev)
     }
     e = cudaMemcpyToSymbol(g_fft_twiddles, host, sizeof host);
     if (e != cudaSuccess) return h3d_set_error(e, "cudaMemcpyToSymbol(g_fft_twiddles)", __FILE__, __LINE__);
+    if ((rc = plane_attrs())) return rc;
     s.ctx_id = id;
     s.ready = true;
     return 0;
+}
+
+// Row (x) and y transform of one z plane per CTA, from the caller's array into
+// the scratch field [z][ky][kx]: the plane's L/2 row pairs are transformed in
+// shared memory, the y transform's first stage takes the split half spectra
+// straight from there and its exchange buffer reuses the rows' (L (L/2+1)
+// elements fit the padded L/2 rows of L).  A plane (10 KB at L = 32, 147 KB at
+// 128) never leaves the SM between the two passes.  At these sizes a call is
+// bound by its chain of launches, each a few microseconds whatever the field's
+// size: this one takes the place of a copy of the input, a row pass and a y
+// pass (48^3: 18.4 us a call with those, 10.9 with this kernel and the z pass).
+// The arithmetic is theirs, operation for operation.
+template <int L> struct PlaneCfg {
+    static constexpr int NH = L / 2 + 1;
+    static constexpr int NT0 = (NH * L / plan_rmax(L) + 31) / 32 * 32;
+    // L = 128: two y butterflies a thread (a CTA of 1040 is not possible)
+    static constexpr int NT = NT0 > 640 ? (NT0 / 2 + 31) / 32 * 32 : NT0;
+    static constexpr size_t SMEM = (size_t)Lay<L, L / 2, true>::elems * sizeof(double2);
+    static_assert(Lay<L, NH, false>::elems <= Lay<L, L / 2, true>::elems, "y exchange buffer");
+};
+template <int L>
+__global__ void __launch_bounds__(PlaneCfg<L>::NT) k_plane_fwd(const double *__restrict__ in, double2 *__restrict__ w,
+                                                              const double2 *__restrict__ tw)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double2 *sm = reinterpret_cast<double2 *>(smraw);
+    constexpr int NT = PlaneCfg<L>::NT, NH = PlaneCfg<L>::NH;
+    using FX = ColFFT<double, L, L / 2, NT, true, true, false>;
+    using FY = ColFFT<double, L, NH, NT, false, true, false>;
+    using LX = typename FX::LY;
+    const double *A = in + (int64_t)blockIdx.x * L * (2 * NH);
+    {
+        double2 v[FX::NIN];
+#pragma unroll
+        for (int i = 0; i < FX::NB0; i++)
+#pragma unroll
+            for (int m = 0; m < FX::R0; m++) {
+                int c, p;
+                if (FX::in_slot(i, m, c, p))
+                    v[i * FX::R0 + m] = make_double2(A[(2 * c) * (2 * NH) + p], A[(2 * c + 1) * (2 * NH) + p]);
+            }
+        // each last-stage butterfly stores at the positions it has read itself
+        FX::run_store(v, sm, tw, [&](int c, int p, double2 z) { sm[LX::idx(c, p)] = z; });
+    }
+    __syncthreads();
+    double2 v[FY::NIN];
+#pragma unroll
+    for (int i = 0; i < FY::NB0; i++)
+#pragma unroll
+        for (int m = 0; m < FY::R0; m++) {
+            int k, y;
+            if (FY::in_slot(i, m, k, y)) {
+                const int c = y >> 1;
+                const double2 zk = sm[LX::idx(c, k)], zm = sm[LX::idx(c, k == 0 ? 0 : L - k)];
+                v[i * FY::R0 + m] = (y & 1) ? make_double2(0.5 * (zk.y + zm.y), -0.5 * (zk.x - zm.x))
+                                            : make_double2(0.5 * (zk.x + zm.x), 0.5 * (zk.y - zm.y));
+            }
+        }
+    __syncthreads();  // every row is read: the buffer turns into the y exchange buffer
+    double2 *W = w + (int64_t)blockIdx.x * L * NH;
+    FY::run_store(v, sm, tw, [&](int k, int p, double2 z) { W[p * NH + k] = z; });
+}
+
+template <int L> int plane_attr()
+{
+    if (PlaneCfg<L>::SMEM <= 48 * 1024) return 0;
+    cudaError_t e = cudaFuncSetAttribute(k_plane_fwd<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PlaneCfg<L>::SMEM);
+    return e == cudaSuccess ? 0 : h3d_set_error(e, "cudaFuncSetAttribute", __FILE__, __LINE__);
 }
 
 template <int L> int run(const DevState &s, const double *in, double *out, cudaStream_t st)
@@ -128,31 +199,11 @@ template <int L> int run(const DevState &s, const double *in, double *out, cudaS
     const int n = L, nh = L / 2 + 1;
     const double2 *tw = s.tw + tw_offset(n);
     double2 *w = s.scratch;
-    cudaError_t e = cudaMemcpyAsync(w, in, sizeof(double2) * (size_t)nh * n * n, cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return h3d_set_error(e, "cudaMemcpyAsync", __FILE__, __LINE__);
-    // the launch shapes of the context path's passes (RowCfg, ColCfg), all
-    // within the default 48 KB of dynamic shared memory, so no attribute call
-    using RC = RowCfg<double, L>;
-    using CY = ColCfg<double, L, true>;
+    k_plane_fwd<L><<<n, PlaneCfg<L>::NT, PlaneCfg<L>::SMEM, st>>>(in, w, tw);
+    // z: out of place into the caller's array, transposed to (kx, kz, ky), with
+    // the launch shape of the context path's pass
     using CZ = ColCfg<double, L, false>;
-    static_assert(RC::SMEM <= 48 * 1024 && CY::SMEM <= 48 * 1024 && CZ::SMEM <= 48 * 1024,
-                  "static transform: shared memory above the default limit");
-    // x: r2c of row pairs, in place (row pitch nh complex = the reference's nx+2 reals)
-    {
-        const int npairs = n * n / 2;
-        k_xr2c<double, L, RC::TC, RC::NT, double><<<(npairs + RC::TC - 1) / RC::TC, RC::NT, RC::SMEM, st>>>(
-            w, 0, nh, npairs, tw, 0);
-    }
-    // y: in place, [z][ky][kx]
-    {
-        IOPlain<double, double, double> io;
-        io.src = w; io.dst = w; io.fs_src = io.fs_dst = 0; io.ncol = nh;
-        io.sa_src = io.sa_dst = nh;
-        io.so_src = io.so_dst = (int64_t)n * nh;
-        dim3 g((nh + CY::TC - 1) / CY::TC, n, 1);
-        k_colfft<double, L, CY::TC, CY::NT, true, IOPlain<double, double, double>><<<g, CY::NT, CY::SMEM, st>>>(io, tw);
-    }
-    // z: out of place into the caller's array, transposed to (kx, kz, ky)
+    static_assert(CZ::SMEM <= 48 * 1024, "static transform: shared memory above the default limit");
     {
         IOPlain<double, double, double> io;
         io.src = w; io.dst = reinterpret_cast<double2 *>(out); io.fs_src = io.fs_dst = 0; io.ncol = nh;
@@ -161,9 +212,17 @@ template <int L> int run(const DevState &s, const double *in, double *out, cudaS
         dim3 g((nh + CZ::TC - 1) / CZ::TC, n, 1);
         k_colfft<double, L, CZ::TC, CZ::NT, true, IOPlain<double, double, double>><<<g, CZ::NT, CZ::SMEM, st>>>(io, tw);
     }
-    e = cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return h3d_set_error(e, "kernel launch", __FILE__, __LINE__);
     return 0;
+}
+
+int plane_attrs()
+{
+    int rc = plane_attr<32>();
+    if (rc == 0) rc = plane_attr<48>();
+    if (rc == 0) rc = plane_attr<64>();
+    return rc ? rc : plane_attr<128>();
 }
 
 }  // namespace
