@@ -31,9 +31,14 @@ template <typename T, int L, int V> struct RowCfgV {
 //       (k_xfused_v2); FP64 at L >= 512 keeps the last physical field in
 //       shared memory between the inverse and forward transforms
 //   14: as 13 with two physical fields in shared memory (FP64), one (FP32)
+// L = 48 (radices 4, 4, 3) has no radix 8 to give a thread eight elements in one
+// butterfly: one radix-4 butterfly a thread and five CTAs per SM at 128
+// registers (eight elements in two butterflies spilled up to 984 bytes; the pass
+// of 32 runs takes 0.087 ms)
 template <typename T, int L> struct RowCfgSmall {
-    static constexpr int TC = L >= 512 ? 1 : 512 / L;
-    static constexpr int NT = L >= 1024 ? 128 : 64;
+    static constexpr int TC = L >= 512 ? 1 : L == 48 ? 8 : 512 / L;
+    static constexpr int NT = L >= 1024 ? 128 : L == 48 ? 96 : 64;
+    static constexpr int MINB = L == 48 ? 5 : (sizeof(T) == 4 ? 384 : 256) / NT;  // CTAs per SM
     static constexpr size_t SMEM = (size_t)Lay<L, TC, true>::elems * sizeof(cx<T>);
 };
 constexpr int kFusedVariants = HIT3D_FUSED_VARIANTS;
@@ -96,7 +101,9 @@ static int xfused_st_L(hit3d_ctx *c, FusedArgs a)
     int per_sm = (int)(233472 / (smem + 1024));
     per_sm = per_sm < MINB ? per_sm : MINB;
     if (per_sm < 1) return h3d_set_error_msg(-1, "fused x pass: stage does not fit in shared memory");
-    const int tiles = (a.npairs + RC::TC - 1) / RC::TC;
+    // the tiles of every run of a batch (one run's alone left a class of 32 runs
+    // of 32^3 with 32 CTAs, 0.29 ms a pass; 0.028 with a full wave)
+    const int tiles = (a.npairs + RC::TC - 1) / RC::TC * (a.nruns > 1 ? a.nruns : 1);
     int grid = c->nsm * per_sm;
     grid = grid < tiles ? grid : tiles;
     k<<<dim3(grid), RC::NT, smem, c->st>>>(a, twid<T>(c));
@@ -128,7 +135,9 @@ static int xfused_v2_L(hit3d_ctx *c, FusedArgs a)
     int per_sm = (int)(233472 / (smem + 1024));
     per_sm = per_sm < MINB ? per_sm : MINB;
     if (per_sm < 1) return h3d_set_error_msg(-1, "fused x pass: stage does not fit in shared memory");
-    const int tiles = (a.npairs + RC::TC - 1) / RC::TC;
+    // the tiles of every run of a batch (one run's alone left a class of 32 runs
+    // of 32^3 with 32 CTAs, 0.29 ms a pass; 0.028 with a full wave)
+    const int tiles = (a.npairs + RC::TC - 1) / RC::TC * (a.nruns > 1 ? a.nruns : 1);
     int grid = c->nsm * per_sm;
     grid = grid < tiles ? grid : tiles;
     k<<<dim3(grid), RC::NT, smem, c->st>>>(a, twid<T>(c));
@@ -145,25 +154,19 @@ template <typename T, template <class> class OP, int L> static int xfused_L(hit3
             using RS = RowCfgSmall<T, L>;
             constexpr int N13 = (sizeof(T) == 8 && L >= 512 && OP<T>::NIN == 3) ? 1 : 0;
             constexpr int N14 = OP<T>::NIN < 3 ? 0 : sizeof(T) == 8 ? 2 : 1;
-            if constexpr (sizeof(T) == 4) {
-                if (c->xcfg == 13) return xfused_v2_L<T, OP, L, 384 / RS::NT, RS, N13>(c, a);
-                return xfused_v2_L<T, OP, L, 384 / RS::NT, RS, N14>(c, a);
-            } else {
-                if (c->xcfg == 13) return xfused_v2_L<T, OP, L, 256 / RS::NT, RS, N13>(c, a);
-                return xfused_v2_L<T, OP, L, 256 / RS::NT, RS, N14>(c, a);
-            }
+            if (c->xcfg == 13) return xfused_v2_L<T, OP, L, RS::MINB, RS, N13>(c, a);
+            return xfused_v2_L<T, OP, L, RS::MINB, RS, N14>(c, a);
         }
         if (c->xcfg == 8) return xfused_st_L<T, OP, L, 3, 2>(c, a);
         if (c->xcfg == 9) return xfused_st_L<T, OP, L, 2, 2>(c, a);
         if (c->xcfg == 10) return xfused_st_L<T, OP, L, 1, sizeof(T) == 4 ? 4 : 3>(c, a);
         if (c->xcfg == 11) {
             using RS = RowCfgSmall<T, L>;  // 256 threads per SM at the full register file
-            return xfused_st_L<T, OP, L, 3, 256 / RS::NT, RS>(c, a);
+            return xfused_st_L<T, OP, L, 3, L == 48 ? RS::MINB : 256 / RS::NT, RS>(c, a);
         }
         if (c->xcfg == 12) {
             using RS = RowCfgSmall<T, L>;
-            if constexpr (sizeof(T) == 4) return xfused_st_L<T, OP, L, 3, 384 / RS::NT, RS>(c, a);  // 168 registers
-            else return xfused_st_L<T, OP, L, 2, 256 / RS::NT, RS>(c, a);
+            return xfused_st_L<T, OP, L, sizeof(T) == 4 ? 3 : 2, RS::MINB, RS>(c, a);  // FP32: 168 registers
         }
         if (c->xcfg == 5) return xfused_ms_L<T, OP, L, 3>(c, a);
         if (c->xcfg == 6) return xfused_ms_L<T, OP, L, 2>(c, a);
