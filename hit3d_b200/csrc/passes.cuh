@@ -758,7 +758,7 @@ H3D_D void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "me
 
 template <typename TS> struct StageRow {
     static constexpr int PER = 16 / (int)sizeof(cx<TS>);  // elements per 16-byte chunk
-    static H3D_HD int chunks(int lim) { return (lim + PER - 1) / PER; }
+    static H3D_HD constexpr int chunks(int lim) { return (lim + PER - 1) / PER; }
 };
 
 template <typename TS, int NIN, int TC, int NT>

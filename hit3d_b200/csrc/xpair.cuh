@@ -1,0 +1,262 @@
+// Fused x passes of the operators with more than three inputs: the scalar
+// fluxes (OpScal: u, v, w, phi -> phi u, phi v, phi w) and the Smagorinsky
+// stress (OpSmag: six strain components -> six stresses).
+//
+// Four or six physical fields do not fit a thread's registers next to the
+// transforms in flight, so the inverse transforms run two at a time and a field
+// leaves the registers before the next pair starts.  Both kernels are a grid of
+// resident CTAs (64 threads, four to an SM in FP64) walking the row pairs, with
+// the next tile's rows brought in by cp.async while the current one is
+// transformed, as k_xfused_st.  What bounds them is what bounds the velocity
+// pass: shared-memory exchanges and FP64 latency at 8 warps per SM; DRAM stays
+// below a third of its rate.
+//
+// In FP64 the last forward stage splits the packed rows in registers
+// (xf_last_split); in FP32 it goes through shared memory (store_split), which
+// keeps the FP32 form's rounding that of the separate passes.
+// Against the register-resident kernel, which held every field of a tile in
+// registers and spilled: scalar fluxes at 256^3 unpruned 0.79 -> 0.41 ms,
+// Smagorinsky stress at 128^3 0.19 -> 0.08 ms.
+#pragma once
+#include "passes.cuh"
+#include "xfused2.cuh"
+
+template <int N> H3D_D void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// the rows (kx < lim, in 16-byte chunks) of NF fields from f0 on, of the TC row
+// pairs at pair0: field f0 + i to dst + i * dstride as [row][rs]; rows of pairs
+// beyond npairs are not copied
+template <typename TS, int NF, int TC, int NT>
+H3D_D void xp_issue(const FusedArgs &a, int f0, cx<TS> *dst, int dstride, int pair0, int nch)
+{
+    constexpr int PER = StageRow<TS>::PER;
+    const int rs = nch * PER;
+#pragma unroll
+    for (int f = 0; f < NF; f++) {
+        const cx<TS> *base = reinterpret_cast<const cx<TS> *>(a.in[f0 + f]) + (int64_t)(2 * pair0) * a.pitch;
+        if constexpr (TC == 1) {
+            if (pair0 < a.npairs)
+#pragma unroll
+                for (int r = 0; r < 2; r++)
+                    for (int ch = threadIdx.x; ch < nch; ch += NT)
+                        cp_async16(dst + f * dstride + r * rs + ch * PER, base + r * a.pitch + ch * PER);
+        } else {
+            const int total = 2 * TC * nch;
+            const DivU32 dch(nch);  // q < total <= 2^16, nch <= 513
+            for (int q = threadIdx.x; q < total; q += NT) {
+                const int r = dch(q), ch = q - r * nch;
+                if (pair0 + r / 2 < a.npairs) cp_async16(dst + f * dstride + r * rs + ch * PER, base + r * a.pitch + ch * PER);
+            }
+        }
+    }
+}
+
+// forward transforms of NF packed fields already in registers, split and stored
+// to a.out[o0 .. o0 + NF); ends with the buffers free
+template <typename T, int L, int TC, int NT, int NF, typename TS>
+H3D_D void xp_forward(const FusedArgs &a, int o0, cx<T> (&in)[NF][ColFFT<T, L, TC, NT, true, true, false>::NIN], cx<T> *sm,
+                      const cx<T> *__restrict__ tw, int pair0, int lim)
+{
+    using FF = RowFFT<T, L, TC, NT, false>;
+    using LY = typename FF::LY;
+    constexpr int E = LY::elems;
+    if constexpr (sizeof(T) == 8) {
+        FF::template run_multi_front<NF>(in, sm, tw);
+        void *outs[NF];
+#pragma unroll
+        for (int f = 0; f < NF; f++) outs[f] = a.out[o0 + f];
+        xf_last_split<T, L, TC, NT, NF, TS>(sm, tw, outs, a.pitch, pair0, a.npairs, lim, (T)0.5);
+    } else {
+        cx<T> out[NF][FF::NOUT];
+        FF::template run_multi<NF>(in, sm, out, tw);
+        __syncthreads();
+#pragma unroll
+        for (int f = 0; f < NF; f++)
+#pragma unroll
+            for (int i = 0; i < FF::NBL; i++)
+#pragma unroll
+                for (int m = 0; m < FF::RL; m++) {
+                    int c, p;
+                    if (FF::out_slot(i, m, c, p)) sm[f * E + LY::idx(c, p)] = out[f][i * FF::RL + m];
+                }
+        __syncthreads();
+#pragma unroll
+        for (int f = 0; f < NF; f++)
+            store_split<T, L, TC, NT, TS>(sm + f * E, reinterpret_cast<cx<TS> *>(a.out[o0 + f]), a.pitch, pair0, a.npairs, lim);
+    }
+    __syncthreads();
+}
+
+// packed inputs of the inverse transforms from the staged rows of two fields
+template <typename T, int L, int TC, int NT, typename TS>
+H3D_D void xp_load2(const FusedArgs &a, const cx<TS> *s0, const cx<TS> *s1, int rs, int pair0, int lim,
+                    cx<T> (&in)[2][ColFFT<T, L, TC, NT, true, false, true>::NIN])
+{
+    using FI = RowFFT<T, L, TC, NT, true>;
+#pragma unroll
+    for (int f = 0; f < 2; f++)
+#pragma unroll
+        for (int i = 0; i < FI::NB0; i++)
+#pragma unroll
+            for (int m = 0; m < FI::R0; m++) {
+                int c, p;
+                if (FI::in_slot(i, m, c, p) && pair0 + c < a.npairs) {
+                    const cx<TS> *A = (f == 0 ? s0 : s1) + 2 * c * rs;
+                    in[f][i * FI::R0 + m] = load_packed<T, L, TS>(A, A + rs, p, lim);
+                } else in[f][i * FI::R0 + m] = mk<T>(0, 0);
+            }
+}
+
+// Scalar fluxes.  Inputs u, v, w, phi (a.in[0..4)), outputs phi u, phi v, phi w.
+// phi and u are inverse-transformed together, then v and w with phi and phi u
+// waiting in registers; the three products go forward in lockstep.  Three
+// exchange buffers and the stage of four fields: 50 KB at 512 elements in FP64.
+template <typename T, int L, int TC, int NT, typename TS, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_xscal(const FusedArgs a, const cx<T> *__restrict__ tw)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    using FI = RowFFT<T, L, TC, NT, true>;
+    using FF = RowFFT<T, L, TC, NT, false>;
+    static_assert(FI::NOUT == FF::NIN, "slot hand-off mismatch");
+    constexpr int NP = FI::NOUT, E = Lay<L, TC, true>::elems;
+    constexpr size_t SOFF = ((size_t)3 * E * sizeof(cx<T>) + 15) / 16 * 16;
+    cx<T> *sm = reinterpret_cast<cx<T> *>(smraw);
+    cx<TS> *st = reinterpret_cast<cx<TS> *>(smraw + SOFF);
+    const T norm = (T)a.norm;
+    const int lim = a.kx_lim > 0 ? a.kx_lim : L / 2 + 1;
+    const int nch = StageRow<TS>::chunks(lim), rs = nch * StageRow<TS>::PER, fst = 2 * TC * rs;
+    const int ntiles = (a.npairs + TC - 1) / TC;
+    if ((int)blockIdx.x < ntiles) xp_issue<TS, 4, TC, NT>(a, 0, st, fst, blockIdx.x * TC, nch);
+    cp_async_commit();
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int pair0 = tile * TC;
+        cx<T> phi[NP], prod[3][NP];
+        cp_async_wait_all();
+        __syncthreads();
+        {
+            cx<T> in[2][FI::NIN], out[2][NP];
+            xp_load2<T, L, TC, NT, TS>(a, st + 3 * fst, st, rs, pair0, lim, in);
+#pragma unroll
+            for (int q = 0; q < NP; q++) out[0][q] = out[1][q] = mk<T>(0, 0);  // slots of idle butterflies
+            FI::template run_multi<2>(in, sm, out, tw);
+#pragma unroll
+            for (int q = 0; q < NP; q++) {
+                phi[q] = mk<T>(out[0][q].x * norm, out[0][q].y * norm);
+                prod[0][q] = mk<T>(phi[q].x * (out[1][q].x * norm), phi[q].y * (out[1][q].y * norm));
+            }
+        }
+        {
+            cx<T> in[2][FI::NIN], out[2][NP];
+            xp_load2<T, L, TC, NT, TS>(a, st + fst, st + 2 * fst, rs, pair0, lim, in);
+#pragma unroll
+            for (int q = 0; q < NP; q++) out[0][q] = out[1][q] = mk<T>(0, 0);
+            __syncthreads();  // the stage and the exchange buffers are read
+            if (tile + (int)gridDim.x < ntiles) xp_issue<TS, 4, TC, NT>(a, 0, st, fst, (tile + gridDim.x) * TC, nch);
+            cp_async_commit();
+            FI::template run_multi<2>(in, sm, out, tw);
+#pragma unroll
+            for (int q = 0; q < NP; q++) {
+                prod[1][q] = mk<T>(phi[q].x * (out[0][q].x * norm), phi[q].y * (out[0][q].y * norm));
+                prod[2][q] = mk<T>(phi[q].x * (out[1][q].x * norm), phi[q].y * (out[1][q].y * norm));
+            }
+        }
+        __syncthreads();  // the exchange buffers are read
+        xp_forward<T, L, TC, NT, 3, TS>(a, 0, prod, sm, tw, pair0, lim);
+    }
+    cp_async_wait_all();
+}
+
+// Smagorinsky stress (OpSmag's arithmetic: nu_t = p0 sqrt(2 S:S), tau = -2 nu_t S).
+// Buffer f holds field f throughout: its staged input rows, the exchanges of its
+// inverse transform, its physical values (each thread at its own slots) and the
+// exchanges of its forward transform; as a pair of fields leaves for HBM the
+// next tile's rows of that pair are copied in.  Six buffers: 55 KB at 512
+// elements in FP64, four CTAs per SM.
+template <typename T, int L, int TC, int NT, typename TS, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_xsmag(const FusedArgs a, const cx<T> *__restrict__ tw)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    using FI = RowFFT<T, L, TC, NT, true>;
+    using FF = RowFFT<T, L, TC, NT, false>;
+    static_assert(FI::NOUT == FF::NIN && sizeof(T) == sizeof(TS), "slot hand-off mismatch");
+    constexpr int NP = FI::NOUT, E = Lay<L, TC, true>::elems;
+    // the staged rows of a pair fit its transform's padded buffer
+    static_assert(2 * StageRow<TS>::chunks(L / 2 + 1) * StageRow<TS>::PER <= L + L / 8 && E * sizeof(cx<T>) % 16 == 0, "stage");
+    using LY = Lay<L, TC, true>;
+    cx<T> *sm = reinterpret_cast<cx<T> *>(smraw);
+    const T norm = (T)a.norm, p0 = (T)a.p0;
+    const int lim = a.kx_lim > 0 ? a.kx_lim : L / 2 + 1;
+    const int nch = StageRow<TS>::chunks(lim), rs = nch * StageRow<TS>::PER;
+    const int ntiles = (a.npairs + TC - 1) / TC;
+#pragma unroll
+    for (int g = 0; g < 3; g++) {
+        if ((int)blockIdx.x < ntiles) xp_issue<TS, 2, TC, NT>(a, 2 * g, sm + 2 * g * E, E, blockIdx.x * TC, nch);
+        cp_async_commit();
+    }
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int pair0 = tile * TC;
+        cx<T> ss[NP];
+#pragma unroll
+        for (int g = 0; g < 3; g++) {
+            cx<T> *b = sm + 2 * g * E;
+            cx<T> in[2][FI::NIN], out[2][NP];
+            if (g == 0) cp_async_wait_group<2>();
+            else if (g == 1) cp_async_wait_group<1>();
+            else cp_async_wait_group<0>();
+            __syncthreads();
+            xp_load2<T, L, TC, NT, TS>(a, b, b + E, rs, pair0, lim, in);
+#pragma unroll
+            for (int q = 0; q < NP; q++) out[0][q] = out[1][q] = mk<T>(0, 0);
+            __syncthreads();  // the staged rows are read: the buffers turn into exchange buffers
+            FI::template run_multi<2>(in, b, out, tw);
+            __syncthreads();  // and into the physical fields
+#pragma unroll
+            for (int i = 0; i < FI::NBL; i++)
+#pragma unroll
+                for (int m = 0; m < FI::RL; m++) {
+                    const int q = i * FI::RL + m;
+                    const cx<T> s0 = mk<T>(out[0][q].x * norm, out[0][q].y * norm), s1 = mk<T>(out[1][q].x * norm, out[1][q].y * norm);
+                    // S11 S12 | S13 S22 | S23 S33, the off-diagonal ones twice
+                    if (g == 0) {
+                        ss[q] = mk<T>(s0.x * s0.x, s0.y * s0.y);
+                        ss[q] = mk<T>(ss[q].x + (T)2 * (s1.x * s1.x), ss[q].y + (T)2 * (s1.y * s1.y));
+                    } else {
+                        ss[q] = mk<T>(ss[q].x + (T)2 * (s0.x * s0.x), ss[q].y + (T)2 * (s0.y * s0.y));
+                        ss[q] = mk<T>(ss[q].x + s1.x * s1.x, ss[q].y + s1.y * s1.y);
+                    }
+                    int c, p;
+                    if (FI::out_slot(i, m, c, p)) {
+                        b[LY::idx(c, p)] = s0;
+                        b[E + LY::idx(c, p)] = s1;
+                    }
+                }
+        }
+#pragma unroll
+        for (int q = 0; q < NP; q++) ss[q] = mk<T>((T)-2 * (sqrt((T)2 * ss[q].x) * p0), (T)-2 * (sqrt((T)2 * ss[q].y) * p0));
+#pragma unroll
+        for (int g = 0; g < 3; g++) {
+            cx<T> *b = sm + 2 * g * E;
+            cx<T> in[2][FF::NIN];
+#pragma unroll
+            for (int i = 0; i < FF::NB0; i++)
+#pragma unroll
+                for (int m = 0; m < FF::R0; m++) {
+                    const int q = i * FF::R0 + m;
+                    int c, p;
+                    in[0][q] = in[1][q] = mk<T>(0, 0);
+                    if (FF::in_slot(i, m, c, p)) {  // the slots the inverse left this thread
+                        const cx<T> s0 = b[LY::idx(c, p)], s1 = b[E + LY::idx(c, p)];
+                        in[0][q] = mk<T>(ss[q].x * s0.x, ss[q].y * s0.y);
+                        in[1][q] = mk<T>(ss[q].x * s1.x, ss[q].y * s1.y);
+                    }
+                }
+            __syncthreads();
+            xp_forward<T, L, TC, NT, 2, TS>(a, 2 * g, in, b, tw, pair0, lim);
+            if (tile + (int)gridDim.x < ntiles) xp_issue<TS, 2, TC, NT>(a, 2 * g, b, E, (tile + gridDim.x) * TC, nch);
+            cp_async_commit();
+        }
+    }
+    cp_async_wait_all();
+}

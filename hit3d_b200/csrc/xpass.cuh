@@ -6,6 +6,7 @@
 #include "launch_cfg.cuh"
 #include "passes.cuh"
 #include "xfused2.cuh"
+#include "xpair.cuh"
 
 // launch-shape variants of the fused x pass (picked by the tuner):
 //   0: 1024/L pairs x 128 threads   1: 2048/L pairs x 128 threads
@@ -145,9 +146,48 @@ static int xfused_v2_L(hit3d_ctx *c, FusedArgs a)
     return 0;
 }
 
+// the operators with more than three inputs (xpair.cuh): one launch shape, the
+// small CTAs of variants 11-14, whatever the variant
+template <typename T, template <class> class OP, int L> static int xpair_L(hit3d_ctx *c, FusedArgs a)
+{
+    using RC = RowCfgSmall<T, L>;
+    constexpr int NIN = OP<T>::NIN, MINB = RC::MINB;
+    static_assert(NIN == 4 || NIN == 6, "scalar fluxes or Smagorinsky stress");
+    for (int f = 0; f < NIN; f++)
+        if (reinterpret_cast<uintptr_t>(a.in[f]) % 16 != 0)
+            return h3d_set_error_msg(-1, "fused x pass: input field not 16-byte aligned");
+    if ((a.pitch * (int64_t)sizeof(cx<T>)) % 16 != 0)
+        return h3d_set_error_msg(-1, "fused x pass: row pitch not a multiple of 16 bytes");
+    if ((int64_t)StageRow<T>::chunks(L / 2 + 1) * StageRow<T>::PER > a.pitch)
+        return h3d_set_error_msg(-1, "fused x pass: row pitch too small for the staged rows");
+    const int tiles = (a.npairs + RC::TC - 1) / RC::TC;
+    auto go = [&](auto k, size_t smax, size_t smem) -> int {
+        H3D_TRY(set_smem(k, smax));
+        int per_sm = (int)(233472 / (smem + 1024));
+        per_sm = per_sm < MINB ? per_sm : MINB;
+        if (per_sm < 1) return h3d_set_error_msg(-1, "fused x pass: stage does not fit in shared memory");
+        int grid = c->nsm * per_sm;
+        grid = grid < tiles ? grid : tiles;
+        k<<<dim3(grid), RC::NT, smem, c->st>>>(a, twid<T>(c));
+        H3D_LAUNCH_CHECK();
+        return 0;
+    };
+    if constexpr (NIN == 4) {
+        auto bytes = [&](int l) {
+            return (3 * RC::SMEM + 15) / 16 * 16 +
+                   (size_t)4 * 2 * RC::TC * StageRow<T>::chunks(l) * StageRow<T>::PER * sizeof(cx<T>);
+        };
+        return go(k_xscal<T, L, RC::TC, RC::NT, T, MINB>, bytes(L / 2 + 1), bytes(a.kx_lim > 0 ? a.kx_lim : L / 2 + 1));
+    } else {
+        return go(k_xsmag<T, L, RC::TC, RC::NT, T, MINB>, 6 * RC::SMEM, 6 * RC::SMEM);
+    }
+}
+
 template <typename T, template <class> class OP, int L> static int xfused_L(hit3d_ctx *c, FusedArgs a)
 {
-    if constexpr (OP<T>::NIN <= 3) {
+    if constexpr (OP<T>::NIN > 3) {
+        return xpair_L<T, OP, L>(c, a);
+    } else {
         if (c->xcfg == 13 || c->xcfg == 14) {
             // 13: FP64 at L >= 512 keeps one physical field in shared memory
             // (registers), the rest none; 14: two (FP64) or one (FP32)
@@ -171,17 +211,17 @@ template <typename T, template <class> class OP, int L> static int xfused_L(hit3
         if (c->xcfg == 5) return xfused_ms_L<T, OP, L, 3>(c, a);
         if (c->xcfg == 6) return xfused_ms_L<T, OP, L, 2>(c, a);
         if (c->xcfg == 7) return xfused_ms_L<T, OP, L, 1, sizeof(T) == 4 ? 4 : 3>(c, a);
-    }
-    if (c->xcfg >= 4) return xfused_reg_L<T, OP, L>(c, a);
-    if constexpr (L >= 128) {
-        switch (c->xcfg) {
-        case 1: return xfused_LV<T, OP, L, 1>(c, a);
-        case 2: return xfused_LV<T, OP, L, 2>(c, a);
-        case 3: return xfused_LV<T, OP, L, 3>(c, a);
-        default: break;
+        if (c->xcfg >= 4) return xfused_reg_L<T, OP, L>(c, a);
+        if constexpr (L >= 128) {
+            switch (c->xcfg) {
+            case 1: return xfused_LV<T, OP, L, 1>(c, a);
+            case 2: return xfused_LV<T, OP, L, 2>(c, a);
+            case 3: return xfused_LV<T, OP, L, 3>(c, a);
+            default: break;
+            }
         }
+        return xfused_LV<T, OP, L, 0>(c, a);
     }
-    return xfused_LV<T, OP, L, 0>(c, a);
 }
 template <typename T, template <class> class OP> int xfused(hit3d_ctx *c, FusedArgs a)
 {
