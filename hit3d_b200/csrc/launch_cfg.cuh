@@ -39,7 +39,5 @@ template <typename T, int L, bool YPASS, int CT> struct ColCfgT {
     static constexpr int NT0 = TC * L / plan_rmax(L);
     static constexpr int NT = CT == 0 ? B::NT : NT0 < 32 ? 32 : NT0 > 512 ? 512 : NT0;
     static constexpr size_t SMEM = (size_t)Lay<L, TC, false>::elems * sizeof(cx<T>);
-    // resident CTAs the register cap allows: the default shape's, or four for
-    // the narrow tiles of up to 256 threads and 56 KB
-    static constexpr int MINB = CT == 1 && NT <= 256 && SMEM <= 56 * 1024 ? 4 : ColMinBlocks<T, L, TC, NT>::value;
+    static constexpr int MINB = ColMinBlocks<T, L, TC, NT>::value;  // resident CTAs the register cap allows
 };
