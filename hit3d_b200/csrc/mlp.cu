@@ -28,12 +28,12 @@ struct hit3d_mlp {
     double delta, inv_norm, inv_norm_p;
     // minibatch scratch for up to cap points
     int64_t cap;
-    float *z, *x, *d, *d4, *lossp, *part, *losses;
+    float *part, *losses;
     int32_t *idx;
     int64_t loss_cap;
 };
 
-static int mlp_smem(const void *k)
+static int mlp_smem(const void *k, size_t bytes = MLP_SMEM)
 {
     static std::mutex mu;
     static std::set<std::pair<const void *, int>> done;
@@ -42,7 +42,7 @@ static int mlp_smem(const void *k)
     std::lock_guard<std::mutex> lk(mu);
     auto key = std::make_pair(k, dev);
     if (done.count(key)) return 0;
-    H3D_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MLP_SMEM));
+    H3D_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     done.insert(key);
     return 0;
 }
@@ -110,8 +110,7 @@ extern "C" int hit3d_mlp_destroy(hit3d_mlp *m)
     cudaSetDevice(m->dev);
     if (m->st) cudaStreamSynchronize(m->st);
     for (void *p : {(void *)m->w, (void *)m->m, (void *)m->v, (void *)m->g, (void *)m->wb, (void *)m->A, (void *)m->tau,
-                    (void *)m->z, (void *)m->x, (void *)m->d, (void *)m->d4, (void *)m->lossp, (void *)m->part,
-                    (void *)m->losses, (void *)m->idx})
+                    (void *)m->part, (void *)m->losses, (void *)m->idx})
         mfree(p);
     if (m->st) cudaStreamDestroy(m->st);
     delete m;
@@ -195,20 +194,14 @@ extern "C" int hit3d_mlp_norms(hit3d_mlp *m, double *out2)
 static int ensure_cap(hit3d_mlp *m, int64_t np)
 {
     if (np <= m->cap) return 0;
-    for (void *p : {(void *)m->z, (void *)m->x, (void *)m->d, (void *)m->d4, (void *)m->lossp, (void *)m->part,
-                    (void *)m->idx})
-        mfree(p);
-    m->z = m->x = m->d = m->d4 = m->lossp = m->part = nullptr;
+    mfree(m->part);
+    mfree(m->idx);
+    m->part = nullptr;
     m->idx = nullptr;
     m->cap = 0;
-    const int64_t nb = (np + MLP_NT - 1) / MLP_NT, nc = (np + WG_C - 1) / WG_C;
-    bool ok = cudaMalloc(&m->z, sizeof(float) * 3 * MLP_H * np) == cudaSuccess &&
-              cudaMalloc(&m->d, sizeof(float) * 3 * MLP_H * np) == cudaSuccess &&
-              cudaMalloc(&m->x, sizeof(float) * MLP_IN * np) == cudaSuccess &&
-              cudaMalloc(&m->d4, sizeof(float) * MLP_OUT * np) == cudaSuccess &&
-              cudaMalloc(&m->lossp, sizeof(float) * nb) == cudaSuccess &&
-              cudaMalloc(&m->part, sizeof(float) * MLP_NPARAM * nc) == cudaSuccess &&
-              cudaMalloc(&m->idx, sizeof(int32_t) * np) == cudaSuccess;
+    const int64_t nc = (np + WG_C - 1) / WG_C;
+    const bool ok = cudaMalloc(&m->part, sizeof(float) * (MLP_NPARAM + 1) * nc) == cudaSuccess &&
+                    cudaMalloc(&m->idx, sizeof(int32_t) * np) == cudaSuccess;
     if (!ok) return h3d_set_error_msg(-4, "hit3d_mlp: out of device memory for the minibatch");
     m->cap = np;
     return 0;
@@ -219,26 +212,19 @@ static MlpBatch batch_args(hit3d_mlp *m, int64_t np, double lam)
     MlpBatch b;
     b.np = np; b.idx = m->idx; b.A = m->A; b.tau = m->tau; b.P = m->P;
     b.delta = (float)m->delta; b.inv_norm = (float)m->inv_norm; b.inv_norm_p = (float)m->inv_norm_p; b.lam = (float)lam;
-    b.z = m->z; b.x = m->x; b.d = m->d; b.d4 = m->d4; b.loss = m->lossp;
+    b.part = m->part;
     return b;
 }
 
 // loss (into dev_loss) and gradient (into m->g) of the minibatch in m->idx
 static int loss_grad(hit3d_mlp *m, int64_t np, double lam, float *dev_loss)
 {
-    M_TRY(mlp_smem((const void *)k_mlp_fwd));
-    M_TRY(mlp_smem((const void *)k_mlp_bwd));
+    M_TRY(mlp_smem((const void *)k_mlp_grad, GS_SMEM));
     const MlpBatch b = batch_args(m, np, lam);
-    const int nb = (int)((np + MLP_NT - 1) / MLP_NT), nc = (int)((np + WG_C - 1) / WG_C);
-    k_mlp_fwd<<<nb, MLP_NT, MLP_SMEM, m->st>>>(b, m->wb);
+    const int nc = (int)((np + WG_C - 1) / WG_C);
+    k_mlp_grad<<<nc, 256, GS_SMEM, m->st>>>(b, m->wb);
     H3D_CHECK(cudaGetLastError());
-    k_sum_partials<<<1, 32, 0, m->st>>>(nb, m->lossp, dev_loss);
-    H3D_CHECK(cudaGetLastError());
-    k_mlp_bwd<<<nb, MLP_NT, MLP_SMEM, m->st>>>(b, m->wb);
-    H3D_CHECK(cudaGetLastError());
-    k_mlp_wgrad_part<<<dim3(nc, 4), 256, 0, m->st>>>(b, m->part);
-    H3D_CHECK(cudaGetLastError());
-    k_mlp_wgrad_sum<<<(MLP_NPARAM + 255) / 256, 256, 0, m->st>>>(nc, m->part, m->g);
+    k_mlp_grad_sum<<<(MLP_NPARAM + 1 + 31) / 32, 256, 0, m->st>>>(nc, m->part, m->g, dev_loss);
     H3D_CHECK(cudaGetLastError());
     return 0;
 }

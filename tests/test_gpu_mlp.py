@@ -37,6 +37,25 @@ def test_loss_and_gradient_match_oracle():
     m.close()
 
 
+@pytest.mark.parametrize("npts", [1, 63, 64, 65, 449, 4097])
+def test_loss_and_gradient_at_chunk_edges(npts):
+    """The gradient kernel's chunks of 64 points and its sum over chunks: one
+    point, a chunk's edges, and chunk counts that the eight groups do not divide.
+    Bounds of test_loss_and_gradient_match_oracle."""
+    A, tau = mo.synthetic_data(1500, seed=11)
+    w = mo.bf16_round(mo.init_params(9)).astype(np.float64)
+    m = _mlp(w)
+    m.set_data(A, tau, DELTA)
+    td = mo.deviatoric(tau)
+    n1, n2 = m.norms()
+    idx = np.random.default_rng(npts).integers(0, 1500, npts).astype(np.int32)
+    loss, g = m.loss_grad(idx, 0.5)
+    ol, og = mo.loss_grad(w, A[:, idx], td[:, idx], DELTA, float(np.float32(n1)), float(np.float32(n2)), 0.5)
+    assert abs(loss - ol) <= 2e-5 * ol
+    assert np.abs(g - og).max() <= 2e-4 * np.abs(og).max()
+    m.close()
+
+
 def test_bf16_weights_are_the_rounded_parameters():
     w = mo.init_params(5).astype(np.float32)
     m = _mlp(w)
