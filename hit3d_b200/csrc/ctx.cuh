@@ -116,6 +116,7 @@ struct hit3d_ctx {
     double2 *W64;        // FP64 scratch (3 fields) for statistics and the transform API
     double2 *sgs;        // FP64 scratch (9 fields) of the subgrid-stress data path, on first use
     double *phys;        // physical u,v,w [3][z][y][x] for particles
+    double2 *shift;      // phase-shift factors exp(i s dx/2), s = -n..3n/2 from entry 0
     double2 *tw64;
     float2 *tw32;
     double *d_fen, *d_part, *d_red, *d_ratio;

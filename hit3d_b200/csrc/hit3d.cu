@@ -50,7 +50,7 @@ static int zinv_LMC(hit3d_ctx *c, int nf, int sfield, const double2 *src, int64_
     IO io;
     io.src = src; io.dst = dst; io.fs_src = src_fs; io.fs_dst = dst_fs;
     io.n = c->n; io.psrc = c->P64; io.pdst = dpitch; io.ncol = c->nh; io.sfield = sfield;
-    io.dx = c->dx;
+    io.sh = c->shift ? c->shift + c->n : nullptr;
     io.k2max = c->k2max;
     io.g = c->zfilt ? c->zfilt : c->gfilt;
     int rows = c->n;
@@ -102,7 +102,6 @@ static int zinv_LM(hit3d_ctx *c, int nf, int sfield, const double2 *src, int64_t
             IOSpec<T, T, PRE_COPY> io;
             io.src = src; io.dst = dst; io.fs_src = src_fs; io.fs_dst = dst_fs;
             io.n = c->n; io.psrc = c->P64; io.pdst = dpitch; io.ncol = c->nh; io.sfield = sfield;
-            io.dx = c->dx;
             int rows = c->n;
             if (c->kc_active >= 0) {
                 io.kl = io.ko = c->kc_active;
@@ -493,6 +492,7 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
     a.flow_type = p.flow_type; a.kfmax = p.kfmax; a.famp = p.famp; a.fenergy = c->d_fen; a.nscal = ns;
     a.kc = c->kc_active;  // pruned state: the updates visit only the kept modes
     a.idle = c->idle_passive;
+    a.shift = c->shift ? c->shift + c->n : nullptr;
     for (int s = 0; s < p.n_scalars; s++) { a.pe[s] = p.nu / p.sc[s]; a.stype[s] = p.scalar_type[s]; }
     for (int j = 0; j < les_nles(p.les_model); j++) {
         // LES fields: Schmidt number one (m_les.f90:372-391), no mean-gradient source
@@ -854,7 +854,7 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
                 } else if (les) {
                     flux = Wf(nprod + 6 + 3 * s);
                 }
-                k_scalar<T><<<pw_grid(c, k_scalar<T>), 256, 0, c->st>>>(a, 0, s, c->dx, Wf(6 + 3 * s), nullptr, c->U,
+                k_scalar<T><<<pw_grid(c, k_scalar<T>), 256, 0, c->st>>>(a, 0, s, Wf(6 + 3 * s), nullptr, c->U,
                                                             c->U + (3 + s) * c->fs64, c->RO + (3 + s) * c->fs64,
                                                             src, flux);
                 H3D_LAUNCH_CHECK();
@@ -867,7 +867,7 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
             }
         } else if (pass == 0) {
             for (int s = 0; s < ns; s++) {
-                k_scalar<T><<<pw_grid(c, k_scalar<T>), 256, 0, c->st>>>(a, 1, s, c->dx, Wf(6 + 3 * s), c->SP + s * c->fs64, c->U,
+                k_scalar<T><<<pw_grid(c, k_scalar<T>), 256, 0, c->st>>>(a, 1, s, Wf(6 + 3 * s), c->SP + s * c->fs64, c->U,
                                                             c->U + (3 + s) * c->fs64, c->RO + (3 + s) * c->fs64);
                 H3D_LAUNCH_CHECK();
             }
@@ -876,12 +876,12 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
         } else {
             for (int s = 0; s < ns; s++) {
                 const cx<T> *rs = (s < p.n_scalars && reac_slot[s] >= 0) ? Wf(reac_slot[s]) : nullptr;
-                k_scalar<T><<<pw_grid(c, k_scalar<T>), 256, 0, c->st>>>(a, 2, s, c->dx, Wf(6 + 3 * s), c->SP + s * c->fs64, c->U,
+                k_scalar<T><<<pw_grid(c, k_scalar<T>), 256, 0, c->st>>>(a, 2, s, Wf(6 + 3 * s), c->SP + s * c->fs64, c->U,
                                                             c->U + (3 + s) * c->fs64, c->RO + (3 + s) * c->fs64,
                                                             nullptr, nullptr, rs);
                 H3D_LAUNCH_CHECK();
             }
-            k_update_vel_ps2<T><<<pw_grid(c, k_update_vel_ps2<T>), 256, 0, c->st>>>(a, c->dx, Wf(0), c->RP, c->U, c->RO);
+            k_update_vel_ps2<T><<<pw_grid(c, k_update_vel_ps2<T>), 256, 0, c->st>>>(a, Wf(0), c->RP, c->U, c->RO);
             H3D_LAUNCH_CHECK();
         }
     }
@@ -1012,6 +1012,15 @@ static int ctx_init(const hit3d_params *p, hit3d_ctx **out, double2 *ext_U, doub
             return rc;
         }
     }
+    if (c->p.dealias == 1) {
+        const int ns = 5 * c->n / 2 + 1;
+        if ((rc = ctx_alloc((void **)&c->shift, sizeof(double2) * (size_t)ns))) {
+            hit3d_gpu_finalize(c);
+            return rc;
+        }
+        k_shift_table<<<(ns + 255) / 256, 256, 0, c->st>>>(c->n, c->dx, c->shift);
+        H3D_LAUNCH_CHECK();
+    }
     if (c->p.precision == 0) c->W64 = reinterpret_cast<double2 *>(c->W);
     else if ((rc = ctx_alloc((void **)&c->W64, f64 * 3))) { hit3d_gpu_finalize(c); return rc; }
     c->pblocks = c->nsm * 2;
@@ -1116,7 +1125,7 @@ extern "C" void hit3d_gpu_finalize(hit3d_ctx *c)
     if (c->sout[1]) cudaFree(c->sout[1]);
     void *ptrs[] = {c->U, c->RO, c->RP, c->SP, c->W, c->phys, c->tw64, c->tw32, c->d_fen, c->d_part,
                     c->d_red, c->d_ratio, c->d_cmax, c->stage, c->d_xyz, c->d_uvw, c->sgs, c->mlp_wb,
-                    c->d_mlp_err, c->d_kmin, c->gfilt, c->pfilt, c->pbuf};
+                    c->d_mlp_err, c->d_kmin, c->gfilt, c->pfilt, c->pbuf, c->shift};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (c->st) cudaStreamDestroy(c->st);

@@ -88,7 +88,7 @@ template <typename T, typename TO, int MODE> struct IOSpec {
     cx<TO> *dst;         // [z][ky][kx] pitch pdst
     int64_t fs_src, fs_dst;
     int n, psrc, pdst, ncol, sfield;
-    double dx;     // grid spacing, for PRE_SHIFT
+    const double2 *sh = nullptr;  // exp(i s dx/2) at entry s = kx + ky + kz, for PRE_SHIFT
     double k2max;  // truncation radius squared, for PRE_TRUNC
     const double2 *g = nullptr;  // test filter transfer function, for PRE_FILT (pitch psrc)
     int kl = -1, ko = -1;  // 2/3-rule pruning of the kz loads and the ky rows
@@ -118,9 +118,8 @@ template <typename T, typename TO, int MODE> struct IOSpec {
         switch (MODE) {
         case PRE_SHIFT: {
             double2 u = U(f, o, c, p);
-            double cs = cos((0.5 * ((kx + ky) + kz)) * dx);
-            double sn = sin((0.5 * ((kx + ky) + kz)) * dx);
-            r = make_double2(u.x * cs - u.y * sn, u.y * cs + u.x * sn);
+            const double2 w = __ldg(sh + (c + kwave(o, n) + kwave(p, n)));
+            r = make_double2(u.x * w.x - u.y * w.y, u.y * w.x + u.x * w.y);
             break;
         }
         case PRE_CURL: {

@@ -136,6 +136,7 @@ struct StepArgs {
     int flow_type, kfmax;
     double famp;
     const double *fenergy;     // device: energy in the forcing band
+    const double2 *shift;      // phase shift: exp(i s dx/2) at entry s = kx + ky + kz
     int nscal;
     double pe[8];
     int stype[8];
@@ -261,6 +262,23 @@ __global__ void k_rhs_vel_ps1(const StepArgs a, const cx<TP> *__restrict__ P, co
     }
 }
 
+// Phase-shift factors exp(i s dx/2) for s = kx + ky + kz = -n .. 3n/2
+// (rhs_velocity.f90:248-257), computed once per run: a double-precision sine and
+// cosine per mode and pass made the shifted z pass and the final update
+// arithmetic-bound (256^3: 0.38 ms for three fields, 0.23 with this table against
+// 0.14 for the plain pass); neighbouring kx read neighbouring entries (10 KB at 256).
+__global__ void k_shift_table(int n, double dx, double2 *__restrict__ t)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > 5 * n / 2) return;
+    const double s = (double)(i - n);
+    t[i] = make_double2(cos((0.5 * s) * dx), sin((0.5 * s) * dx));
+}
+H3D_D double2 shift_at(const double2 *__restrict__ t, const ModeIdx &m, int n)
+{
+    return __ldg(t + (m.kx + kwave(m.kyi, n) + kwave(m.kzi, n)));
+}
+
 // shift back by exp(-i k.delta) (rhs_velocity.f90:276-278)
 H3D_D double2 shift_back(double2 v, double cs, double sn)
 {
@@ -270,7 +288,7 @@ H3D_D double2 shift_back(double2 v, double cs, double sn)
 // phase shift, second half (rhs_velocity.f90:242-408) + forcing + AB2 + pressure.
 // Q: six shifted product spectra [u+u+ u+v+ u+w+ v+v+ v+w+ w+w+]
 template <typename TP>
-__global__ void k_update_vel_ps2(const StepArgs a, double dx, const cx<TP> *__restrict__ Q,
+__global__ void k_update_vel_ps2(const StepArgs a, const cx<TP> *__restrict__ Q,
                                  const double2 *__restrict__ RP, double2 *__restrict__ U, double2 *__restrict__ RO)
 {
     const int64_t nm = (int64_t)a.n * a.n * a.nh;
@@ -283,7 +301,8 @@ __global__ void k_update_vel_ps2(const StepArgs a, double dx, const cx<TP> *__re
         double2 r[3];
         double kx = m.ax, ky = m.ay, kz = m.az;
         if (m.ialias < 2) {
-            double cs = cos((0.5 * ((kx + ky) + kz)) * dx), sn = sin((0.5 * ((kx + ky) + kz)) * dx);
+            const double2 w = shift_at(a.shift, m, a.n);
+            const double cs = w.x, sn = w.y;
             r[0] = RP[o]; r[1] = RP[o + a.fs]; r[2] = RP[o + 2 * a.fs];
             double2 A = shift_back(ld2<TP>(Q, po), cs, sn);                // u+u+
             r[0].x = r[0].x + 0.5 * kx * A.y; r[0].y = r[0].y - 0.5 * kx * A.x;
@@ -325,7 +344,7 @@ template <typename TP>
 // LS, LF (optional, dynamic localization model): spectra of the k_sgs source
 // 2 nu_t S:S - k^(3/2)/Delta and of the three fluxes nu_t dk/dx_i, added to the
 // RHS where ialias == 0 as LS + i k . LF (m_les.f90:1540-1546, 1609-1615, 1080-1086)
-__global__ void k_scalar(const StepArgs a, int mode, int s, double dx, const cx<TP> *__restrict__ P,
+__global__ void k_scalar(const StepArgs a, int mode, int s, const cx<TP> *__restrict__ P,
                          double2 *__restrict__ SP, const double2 *__restrict__ Uvel, double2 *__restrict__ PHI,
                          double2 *__restrict__ RO, const cx<TP> *__restrict__ LS = nullptr,
                          const cx<TP> *__restrict__ LF = nullptr, const cx<TP> *__restrict__ RS = nullptr)
@@ -368,7 +387,8 @@ __global__ void k_scalar(const StepArgs a, int mode, int s, double dx, const cx<
         } else {
             if (m.ialias > 1) r = make_double2(0.0, 0.0);
             else {
-                double cs = cos((0.5 * ((kx + ky) + kz)) * dx), sn = sin((0.5 * ((kx + ky) + kz)) * dx);
+                const double2 w = shift_at(a.shift, m, a.n);
+                const double cs = w.x, sn = w.y;
                 double2 a1 = shift_back(pu, cs, sn), a2 = shift_back(pv, cs, sn), a3 = shift_back(pw, cs, sn);
                 r = make_double2(+0.5 * (kx * a1.y + ky * a2.y + kz * a3.y), -0.5 * (kx * a1.x + ky * a2.x + kz * a3.x));
                 double2 sp = SP[o];
