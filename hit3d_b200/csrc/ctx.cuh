@@ -103,6 +103,16 @@ struct Randu {
 
 constexpr int kCopyStreams = 2;  // copy streams per direction of hit3d_gpu_step_host (4 measured slower)
 
+// everything a step's launches depend on: a recorded step (hit3d_ctx::sg) is
+// replayed only while all of it is what it was at the recording
+struct StepKey {
+    hit3d_params p;
+    int32_t es, int_scalars, idle_passive, xcfg, ctile, kc, pscheme, mlp_clip, mlp_kernel, pad;
+    int64_t np;
+    double mlp_delta;
+    const void *ptr[6];
+};
+
 struct hit3d_ctx {
     hit3d_params p;
     int n, nh, P64, P32, nsc, dev, kmax, nsm;
@@ -161,6 +171,13 @@ struct hit3d_ctx {
     double2 *sin, *sout[2];  // one input staging set, two output sets used in turn
     int nstage_io;           // fields each staging set holds
     cudaEvent_t ev_in_ready, ev_in_free, ev_out_ready, ev_out_free[2];
+    // one Adams-Bashforth step recorded as a graph (grids up to 128), its key,
+    // its kernels, and the steps taken with the current key
+    cudaGraphExec_t sg;
+    StepKey sg_key;
+    int64_t sg_kernels;
+    int sg_seen;
+    unsigned long long *h_words;  // pinned: the Courant maximum and the error word of a call
     int ext_bufs;        // U, RO and W belong to a batch's slab
     int ctile;           // column-tile shape of the plain strided passes (ColCfgT), grids up to 512
     // while a batch class is being stepped through this context (its first

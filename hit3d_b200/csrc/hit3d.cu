@@ -904,6 +904,7 @@ static int ctx_alloc(void **p, size_t bytes)
 // and work fields borrowed from a batch's slab instead of allocated here (the
 // context does not free them).
 static int ctx_init(const hit3d_params *p, hit3d_ctx **out, double2 *ext_U, double2 *ext_RO, void *ext_W);
+static void drop_step_graph(hit3d_ctx *c);
 
 extern "C" int hit3d_gpu_init(const hit3d_params *p, hit3d_ctx **out)
 {
@@ -1099,6 +1100,8 @@ extern "C" void hit3d_gpu_finalize(hit3d_ctx *c)
     if (!c) return;
     cudaSetDevice(c->dev);
     if (c->st) cudaStreamSynchronize(c->st);
+    drop_step_graph(c);
+    if (c->h_words) cudaFreeHost(c->h_words);
     if (c->W64 && c->W64 != c->W) cudaFree(c->W64);
     if (c->ext_bufs) c->U = c->RO = nullptr, c->W = nullptr;  // a batch's slab
     if (c->cs_h2d) {
@@ -1482,6 +1485,83 @@ static bool chain_ok(const hit3d_ctx *c)
     return c->fuse_update && c->p.dealias == 0 && c->p.les_model == 0 && c->bruns == 0;
 }
 
+// A step of a grid up to 128 is 7 to 40 launches of a few microseconds each, and
+// issuing them takes the host longer than the GPU needs (64^3 decaying, 20 calls
+// of one step and a download: 1.33 ms issued one by one, 1.07 replayed; 128^3
+// Smagorinsky, 50 steps: 18.0 -> 16.9 ms).  After kGraphAfter Adams-Bashforth
+// steps with one key the step is recorded, and later steps with the same key
+// replay it with one launch; any change of the key drops the recording.  Below
+// kGraphAfter a run of a few steps would not earn back the recording (about ten
+// steps' saving); above 128 the kernels are long enough to hide their launches.
+constexpr int kGraphMaxN = 128, kGraphAfter = 4;
+
+static StepKey step_key(const hit3d_ctx *c, int es)
+{
+    StepKey k;
+    memset(&k, 0, sizeof k);
+    k.p = c->p;
+    k.es = es;
+    k.int_scalars = c->int_scalars;
+    k.idle_passive = c->idle_passive;
+    k.xcfg = c->xcfg;
+    k.ctile = c->ctile;
+    k.kc = (c->prune_on && c->pruned && c->p.dealias == 0) ? c->n / 3 : -1;
+    k.pscheme = c->pscheme;
+    k.mlp_clip = c->mlp_clip;
+    k.mlp_kernel = c->mlp_kernel;
+    k.np = c->np;
+    k.mlp_delta = c->mlp_delta;
+    const void *ptr[6] = {c->phys, c->d_xyz, c->d_uvw, c->mlp_wb, c->pfilt, c->pbuf};
+    memcpy(k.ptr, ptr, sizeof ptr);
+    return k;
+}
+static void drop_step_graph(hit3d_ctx *c)
+{
+    if (c->sg) cudaGraphExecDestroy(c->sg);
+    c->sg = nullptr;
+    c->sg_seen = 0;
+}
+// record one Adams-Bashforth step; a recording that cannot be made leaves the
+// steps to be issued one by one (sg_seen far below zero)
+static int record_step(hit3d_ctx *c, int es)
+{
+    const int64_t n0 = c->nlaunch;
+    H3D_CHECK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
+    const int rc = c->p.precision == 0 ? step_once<double>(c, 0, es) : step_once<float>(c, 0, es);
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamEndCapture(c->st, &g);
+    if (rc == 0 && e == cudaSuccess) e = cudaGraphInstantiate(&c->sg, g, 0);
+    if (g) cudaGraphDestroy(g);
+    c->sg_kernels = c->nlaunch - n0;
+    c->nlaunch = n0;
+    if (rc != 0 || e != cudaSuccess) {
+        (void)cudaGetLastError();
+        c->sg = nullptr;
+        c->sg_seen = INT32_MIN / 2;
+    }
+    return 0;
+}
+// one step: euler_v, euler_s as step_once; Adams-Bashforth steps of small grids
+// through the recorded graph
+static int take_step(hit3d_ctx *c, int ev, int es, bool zin, bool zout)
+{
+    if (c->n <= kGraphMaxN && !ev && !zin && !zout && c->bruns == 0) {
+        const StepKey k = step_key(c, es);
+        if (memcmp(&k, &c->sg_key, sizeof k) != 0) {
+            drop_step_graph(c);
+            c->sg_key = k;
+        }
+        if (!c->sg && ++c->sg_seen > kGraphAfter) H3D_TRY(record_step(c, es));
+        if (c->sg) {
+            H3D_CHECK(cudaGraphLaunch(c->sg, c->st));
+            c->nlaunch += c->sg_kernels;
+            return 0;
+        }
+    }
+    return c->p.precision == 0 ? step_once<double>(c, ev, es, nullptr, zin, zout)
+                               : step_once<float>(c, ev, es, nullptr, zin, zout);
+}
+
 extern "C" int hit3d_gpu_step(hit3d_ctx *c, int32_t nsteps, int32_t *fov, int32_t *fos, double *courant)
 {
     if (!c) return h3d_set_error_msg(-1, "null context");
@@ -1494,9 +1574,7 @@ extern "C" int hit3d_gpu_step(hit3d_ctx *c, int32_t nsteps, int32_t *fov, int32_
     const bool chain = chain_ok(c);
     for (int it = 0; it < nsteps; it++) {
         const bool zin = chain && it > 0, zout = chain && it + 1 < nsteps;
-        int rc = c->p.precision == 0 ? step_once<double>(c, ev, es, nullptr, zin, zout)
-                                     : step_once<float>(c, ev, es, nullptr, zin, zout);
-        if (rc) return rc;
+        H3D_TRY(take_step(c, ev, es, zin, zout));
         ev = 0;
         if (c->int_scalars) es = 0;
     }
@@ -1510,8 +1588,9 @@ extern "C" int hit3d_gpu_step(hit3d_ctx *c, int32_t nsteps, int32_t *fov, int32_
     }
     if (nsteps > 0) {
         // the Courant maximum and the error word in one read
-        unsigned long long words[2] = {0, 0};
-        H3D_CHECK(cudaMemcpyAsync(words, c->d_cmax, sizeof words, cudaMemcpyDeviceToHost, c->st));
+        if (!c->h_words) H3D_CHECK(cudaMallocHost((void **)&c->h_words, 2 * sizeof(unsigned long long)));
+        unsigned long long *words = c->h_words;
+        H3D_CHECK(cudaMemcpyAsync(words, c->d_cmax, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->st));
         H3D_CHECK(cudaStreamSynchronize(c->st));
         int derr = 0;
         memcpy(&derr, &words[1], sizeof derr);
