@@ -11,9 +11,9 @@
 // pass: shared-memory exchanges and FP64 latency at 8 warps per SM; DRAM stays
 // below a third of its rate.
 //
-// In FP64 the last forward stage splits the packed rows in registers
-// (xf_last_split); in FP32 it goes through shared memory (store_split), which
-// keeps the FP32 form's rounding that of the separate passes.
+// FP64 only: the FP32 form keeps the register-resident kernel, whose rounding its
+// runs repeat (the same operations contracted otherwise differ by 2e-8 after a few
+// steps).
 // Against the register-resident kernel, which held every field of a tile in
 // registers and spilled: scalar fluxes at 256^3 unpruned 0.79 -> 0.41 ms,
 // Smagorinsky stress at 128^3 0.19 -> 0.08 ms.
@@ -58,32 +58,11 @@ H3D_D void xp_forward(const FusedArgs &a, int o0, cx<T> (&in)[NF][ColFFT<T, L, T
                       const cx<T> *__restrict__ tw, int pair0, int lim)
 {
     using FF = RowFFT<T, L, TC, NT, false>;
-    using LY = typename FF::LY;
-    constexpr int E = LY::elems;
-    if constexpr (sizeof(T) == 8) {
-        FF::template run_multi_front<NF>(in, sm, tw);
-        void *outs[NF];
+    FF::template run_multi_front<NF>(in, sm, tw);
+    void *outs[NF];
 #pragma unroll
-        for (int f = 0; f < NF; f++) outs[f] = a.out[o0 + f];
-        xf_last_split<T, L, TC, NT, NF, TS>(sm, tw, outs, a.pitch, pair0, a.npairs, lim, (T)0.5);
-    } else {
-        cx<T> out[NF][FF::NOUT];
-        FF::template run_multi<NF>(in, sm, out, tw);
-        __syncthreads();
-#pragma unroll
-        for (int f = 0; f < NF; f++)
-#pragma unroll
-            for (int i = 0; i < FF::NBL; i++)
-#pragma unroll
-                for (int m = 0; m < FF::RL; m++) {
-                    int c, p;
-                    if (FF::out_slot(i, m, c, p)) sm[f * E + LY::idx(c, p)] = out[f][i * FF::RL + m];
-                }
-        __syncthreads();
-#pragma unroll
-        for (int f = 0; f < NF; f++)
-            store_split<T, L, TC, NT, TS>(sm + f * E, reinterpret_cast<cx<TS> *>(a.out[o0 + f]), a.pitch, pair0, a.npairs, lim);
-    }
+    for (int f = 0; f < NF; f++) outs[f] = a.out[o0 + f];
+    xf_last_split<T, L, TC, NT, NF, TS>(sm, tw, outs, a.pitch, pair0, a.npairs, lim, (T)0.5);
     __syncthreads();
 }
 

@@ -146,8 +146,8 @@ static int xfused_v2_L(hit3d_ctx *c, FusedArgs a)
     return 0;
 }
 
-// the operators with more than three inputs (xpair.cuh): one launch shape, the
-// small CTAs of variants 11-14, whatever the variant
+// the operators with more than three inputs in FP64 (xpair.cuh): one launch shape,
+// the small CTAs of variants 11-14, whatever the variant
 template <typename T, template <class> class OP, int L> static int xpair_L(hit3d_ctx *c, FusedArgs a)
 {
     using RC = RowCfgSmall<T, L>;
@@ -185,32 +185,34 @@ template <typename T, template <class> class OP, int L> static int xpair_L(hit3d
 
 template <typename T, template <class> class OP, int L> static int xfused_L(hit3d_ctx *c, FusedArgs a)
 {
-    if constexpr (OP<T>::NIN > 3) {
+    if constexpr (OP<T>::NIN > 3 && sizeof(T) == 8) {
         return xpair_L<T, OP, L>(c, a);
     } else {
-        if (c->xcfg == 13 || c->xcfg == 14) {
-            // 13: FP64 at L >= 512 keeps one physical field in shared memory
-            // (registers), the rest none; 14: two (FP64) or one (FP32)
-            using RS = RowCfgSmall<T, L>;
-            constexpr int N13 = (sizeof(T) == 8 && L >= 512 && OP<T>::NIN == 3) ? 1 : 0;
-            constexpr int N14 = OP<T>::NIN < 3 ? 0 : sizeof(T) == 8 ? 2 : 1;
-            if (c->xcfg == 13) return xfused_v2_L<T, OP, L, RS::MINB, RS, N13>(c, a);
-            return xfused_v2_L<T, OP, L, RS::MINB, RS, N14>(c, a);
+        if constexpr (OP<T>::NIN <= 3) {
+            if (c->xcfg == 13 || c->xcfg == 14) {
+                // 13: FP64 at L >= 512 keeps one physical field in shared memory
+                // (registers), the rest none; 14: two (FP64) or one (FP32)
+                using RS = RowCfgSmall<T, L>;
+                constexpr int N13 = (sizeof(T) == 8 && L >= 512 && OP<T>::NIN == 3) ? 1 : 0;
+                constexpr int N14 = OP<T>::NIN < 3 ? 0 : sizeof(T) == 8 ? 2 : 1;
+                if (c->xcfg == 13) return xfused_v2_L<T, OP, L, RS::MINB, RS, N13>(c, a);
+                return xfused_v2_L<T, OP, L, RS::MINB, RS, N14>(c, a);
+            }
+            if (c->xcfg == 8) return xfused_st_L<T, OP, L, 3, 2>(c, a);
+            if (c->xcfg == 9) return xfused_st_L<T, OP, L, 2, 2>(c, a);
+            if (c->xcfg == 10) return xfused_st_L<T, OP, L, 1, sizeof(T) == 4 ? 4 : 3>(c, a);
+            if (c->xcfg == 11) {
+                using RS = RowCfgSmall<T, L>;  // 256 threads per SM at the full register file
+                return xfused_st_L<T, OP, L, 3, L == 48 ? RS::MINB : 256 / RS::NT, RS>(c, a);
+            }
+            if (c->xcfg == 12) {
+                using RS = RowCfgSmall<T, L>;
+                return xfused_st_L<T, OP, L, sizeof(T) == 4 ? 3 : 2, RS::MINB, RS>(c, a);  // FP32: 168 registers
+            }
+            if (c->xcfg == 5) return xfused_ms_L<T, OP, L, 3>(c, a);
+            if (c->xcfg == 6) return xfused_ms_L<T, OP, L, 2>(c, a);
+            if (c->xcfg == 7) return xfused_ms_L<T, OP, L, 1, sizeof(T) == 4 ? 4 : 3>(c, a);
         }
-        if (c->xcfg == 8) return xfused_st_L<T, OP, L, 3, 2>(c, a);
-        if (c->xcfg == 9) return xfused_st_L<T, OP, L, 2, 2>(c, a);
-        if (c->xcfg == 10) return xfused_st_L<T, OP, L, 1, sizeof(T) == 4 ? 4 : 3>(c, a);
-        if (c->xcfg == 11) {
-            using RS = RowCfgSmall<T, L>;  // 256 threads per SM at the full register file
-            return xfused_st_L<T, OP, L, 3, L == 48 ? RS::MINB : 256 / RS::NT, RS>(c, a);
-        }
-        if (c->xcfg == 12) {
-            using RS = RowCfgSmall<T, L>;
-            return xfused_st_L<T, OP, L, sizeof(T) == 4 ? 3 : 2, RS::MINB, RS>(c, a);  // FP32: 168 registers
-        }
-        if (c->xcfg == 5) return xfused_ms_L<T, OP, L, 3>(c, a);
-        if (c->xcfg == 6) return xfused_ms_L<T, OP, L, 2>(c, a);
-        if (c->xcfg == 7) return xfused_ms_L<T, OP, L, 1, sizeof(T) == 4 ? 4 : 3>(c, a);
         if (c->xcfg >= 4) return xfused_reg_L<T, OP, L>(c, a);
         if constexpr (L >= 128) {
             switch (c->xcfg) {
