@@ -15,7 +15,7 @@
 // runs repeat (the same operations contracted otherwise differ by 2e-8 after a few
 // steps).
 // Against the register-resident kernel, which held every field of a tile in
-// registers and spilled: scalar fluxes at 256^3 unpruned 0.79 -> 0.41 ms,
+// registers and spilled: scalar fluxes at 256^3 unpruned 0.79 -> 0.36 ms,
 // Smagorinsky stress at 128^3 0.19 -> 0.08 ms.
 #pragma once
 #include "passes.cuh"
@@ -88,52 +88,70 @@ H3D_D void xp_load2(const FusedArgs &a, const cx<TS> *s0, const cx<TS> *s1, int 
 
 // Scalar fluxes.  Inputs u, v, w, phi (a.in[0..4)), outputs phi u, phi v, phi w.
 // phi and u are inverse-transformed together, then v and w with phi and phi u
-// waiting in registers; the three products go forward in lockstep.  Three
-// exchange buffers and the stage of four fields: 50 KB at 512 elements in FP64.
+// waiting in registers; the three products go forward in lockstep.  Five buffers,
+// 46 KB at 512 elements in FP64: the rows of phi and u arrive in buffers 3 and 4
+// (their exchange buffers) while the previous tile's products go forward in 0, 1
+// and 2, those of v and w in 1 and 2 while phi and u are transformed, so that
+// every copy overlaps a transform and four CTAs share an SM.  (With a stage of
+// its own for all four fields an unpruned tile left room for three CTAs.)
 template <typename T, int L, int TC, int NT, typename TS, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_xscal(const FusedArgs a, const cx<T> *__restrict__ tw)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     using FI = RowFFT<T, L, TC, NT, true>;
     using FF = RowFFT<T, L, TC, NT, false>;
-    static_assert(FI::NOUT == FF::NIN, "slot hand-off mismatch");
+    static_assert(FI::NOUT == FF::NIN && sizeof(T) == sizeof(TS), "slot hand-off mismatch");
     constexpr int NP = FI::NOUT, E = Lay<L, TC, true>::elems;
-    constexpr size_t SOFF = ((size_t)3 * E * sizeof(cx<T>) + 15) / 16 * 16;
+    // the staged rows of a pair fit its transform's padded buffer
+    static_assert(2 * StageRow<TS>::chunks(L / 2 + 1) * StageRow<TS>::PER <= L + L / 8 && E * sizeof(cx<T>) % 16 == 0, "stage");
     cx<T> *sm = reinterpret_cast<cx<T> *>(smraw);
-    cx<TS> *st = reinterpret_cast<cx<TS> *>(smraw + SOFF);
+    cx<T> *bp = sm + 3 * E, *bv = sm + E;  // phi and u; v and w
     const T norm = (T)a.norm;
     const int lim = a.kx_lim > 0 ? a.kx_lim : L / 2 + 1;
-    const int nch = StageRow<TS>::chunks(lim), rs = nch * StageRow<TS>::PER, fst = 2 * TC * rs;
+    const int nch = StageRow<TS>::chunks(lim), rs = nch * StageRow<TS>::PER;
     const int ntiles = (a.npairs + TC - 1) / TC;
-    if ((int)blockIdx.x < ntiles) xp_issue<TS, 4, TC, NT>(a, 0, st, fst, blockIdx.x * TC, nch);
-    cp_async_commit();
+    auto issue_phi_u = [&](int tile) {
+        if (tile < ntiles) {
+            xp_issue<TS, 1, TC, NT>(a, 3, bp, E, tile * TC, nch);
+            xp_issue<TS, 1, TC, NT>(a, 0, bp + E, E, tile * TC, nch);
+        }
+        cp_async_commit();
+    };
+    auto issue_v_w = [&](int tile) {
+        if (tile < ntiles) xp_issue<TS, 2, TC, NT>(a, 1, bv, E, tile * TC, nch);
+        cp_async_commit();
+    };
+    issue_phi_u(blockIdx.x);
+    issue_v_w(blockIdx.x);
 #pragma unroll 1
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int pair0 = tile * TC;
         cx<T> phi[NP], prod[3][NP];
-        cp_async_wait_all();
+        cp_async_wait_group<1>();
         __syncthreads();
         {
             cx<T> in[2][FI::NIN], out[2][NP];
-            xp_load2<T, L, TC, NT, TS>(a, st + 3 * fst, st, rs, pair0, lim, in);
+            xp_load2<T, L, TC, NT, TS>(a, bp, bp + E, rs, pair0, lim, in);
 #pragma unroll
             for (int q = 0; q < NP; q++) out[0][q] = out[1][q] = mk<T>(0, 0);  // slots of idle butterflies
-            FI::template run_multi<2>(in, sm, out, tw);
+            __syncthreads();  // the staged rows are read: the buffers turn into exchange buffers
+            FI::template run_multi<2>(in, bp, out, tw);
 #pragma unroll
             for (int q = 0; q < NP; q++) {
                 phi[q] = mk<T>(out[0][q].x * norm, out[0][q].y * norm);
                 prod[0][q] = mk<T>(phi[q].x * (out[1][q].x * norm), phi[q].y * (out[1][q].y * norm));
             }
         }
+        cp_async_wait_group<0>();
+        __syncthreads();  // v and w have arrived, the exchange buffers of phi and u are read
         {
             cx<T> in[2][FI::NIN], out[2][NP];
-            xp_load2<T, L, TC, NT, TS>(a, st + fst, st + 2 * fst, rs, pair0, lim, in);
+            xp_load2<T, L, TC, NT, TS>(a, bv, bv + E, rs, pair0, lim, in);
 #pragma unroll
             for (int q = 0; q < NP; q++) out[0][q] = out[1][q] = mk<T>(0, 0);
-            __syncthreads();  // the stage and the exchange buffers are read
-            if (tile + (int)gridDim.x < ntiles) xp_issue<TS, 4, TC, NT>(a, 0, st, fst, (tile + gridDim.x) * TC, nch);
-            cp_async_commit();
-            FI::template run_multi<2>(in, sm, out, tw);
+            __syncthreads();
+            issue_phi_u(tile + (int)gridDim.x);
+            FI::template run_multi<2>(in, bv, out, tw);
 #pragma unroll
             for (int q = 0; q < NP; q++) {
                 prod[1][q] = mk<T>(phi[q].x * (out[0][q].x * norm), phi[q].y * (out[0][q].y * norm));
@@ -142,6 +160,7 @@ __global__ void __launch_bounds__(NT, MINB) k_xscal(const FusedArgs a, const cx<
         }
         __syncthreads();  // the exchange buffers are read
         xp_forward<T, L, TC, NT, 3, TS>(a, 0, prod, sm, tw, pair0, lim);
+        issue_v_w(tile + (int)gridDim.x);
     }
     cp_async_wait_all();
 }

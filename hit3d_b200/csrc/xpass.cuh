@@ -161,8 +161,8 @@ template <typename T, template <class> class OP, int L> static int xpair_L(hit3d
     if ((int64_t)StageRow<T>::chunks(L / 2 + 1) * StageRow<T>::PER > a.pitch)
         return h3d_set_error_msg(-1, "fused x pass: row pitch too small for the staged rows");
     const int tiles = (a.npairs + RC::TC - 1) / RC::TC;
-    auto go = [&](auto k, size_t smax, size_t smem) -> int {
-        H3D_TRY(set_smem(k, smax));
+    auto go = [&](auto k, size_t smem) -> int {
+        H3D_TRY(set_smem(k, smem));
         int per_sm = (int)(233472 / (smem + 1024));
         per_sm = per_sm < MINB ? per_sm : MINB;
         if (per_sm < 1) return h3d_set_error_msg(-1, "fused x pass: stage does not fit in shared memory");
@@ -172,15 +172,8 @@ template <typename T, template <class> class OP, int L> static int xpair_L(hit3d
         H3D_LAUNCH_CHECK();
         return 0;
     };
-    if constexpr (NIN == 4) {
-        auto bytes = [&](int l) {
-            return (3 * RC::SMEM + 15) / 16 * 16 +
-                   (size_t)4 * 2 * RC::TC * StageRow<T>::chunks(l) * StageRow<T>::PER * sizeof(cx<T>);
-        };
-        return go(k_xscal<T, L, RC::TC, RC::NT, T, MINB>, bytes(L / 2 + 1), bytes(a.kx_lim > 0 ? a.kx_lim : L / 2 + 1));
-    } else {
-        return go(k_xsmag<T, L, RC::TC, RC::NT, T, MINB>, 6 * RC::SMEM, 6 * RC::SMEM);
-    }
+    if constexpr (NIN == 4) return go(k_xscal<T, L, RC::TC, RC::NT, T, MINB>, 5 * RC::SMEM);
+    else return go(k_xsmag<T, L, RC::TC, RC::NT, T, MINB>, 6 * RC::SMEM);
 }
 
 template <typename T, template <class> class OP, int L> static int xfused_L(hit3d_ctx *c, FusedArgs a)
