@@ -131,8 +131,10 @@ struct hit3d_ctx {
     float2 *tw32;
     double *d_fen, *d_part, *d_red, *d_ratio;
     unsigned long long *d_cmax;  // [0]: Courant maximum (bits of a double >= 0); [1]: the error word d_err
+    unsigned long long *zcmax;  // set while the z pass that clears the Courant maximum is issued
     int *d_err;          // device error word: bit 1 = a fused x pass gave up waiting for its input stage
-    double2 *stage;      // one field in the reference layout
+    double2 *stage;      // nstage fields in the reference layout: every state field up to 128^3, else one
+    int nstage;
     double *d_xyz, *d_uvw;
     int64_t np;
     int pscheme;

@@ -1,6 +1,7 @@
 // C-ABI of the B200 pseudospectral step (declared in include/hit3d_gpu.h):
 // device state, transform launchers dispatched on the grid size, the time step
 // pipeline, statistics, initial conditions and particles.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -51,6 +52,7 @@ static int zinv_LMC(hit3d_ctx *c, int nf, int sfield, const double2 *src, int64_
     io.src = src; io.dst = dst; io.fs_src = src_fs; io.fs_dst = dst_fs;
     io.n = c->n; io.psrc = c->P64; io.pdst = dpitch; io.ncol = c->nh; io.sfield = sfield;
     io.sh = c->shift ? c->shift + c->n : nullptr;
+    io.zero = c->zcmax;
     io.k2max = c->k2max;
     io.g = c->zfilt ? c->zfilt : c->gfilt;
     int rows = c->n;
@@ -102,6 +104,7 @@ static int zinv_LM(hit3d_ctx *c, int nf, int sfield, const double2 *src, int64_t
             IOSpec<T, T, PRE_COPY> io;
             io.src = src; io.dst = dst; io.fs_src = src_fs; io.fs_dst = dst_fs;
             io.n = c->n; io.psrc = c->P64; io.pdst = dpitch; io.ncol = c->nh; io.sfield = sfield;
+            io.zero = c->zcmax;
             int rows = c->n;
             if (c->kc_active >= 0) {
                 io.kl = io.ko = c->kc_active;
@@ -571,14 +574,20 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
     for (int pass = 0; pass < npass; pass++) {
         const int mode = pass == 0 ? PRE_COPY : PRE_SHIFT;
         MARK(0);
-        if (!(zin && pass == 0)) H3D_TRY(zinv<T>(c, 3, mode, 0, c->U, c->fs64, Wf(0), wfs, wp));
+        if (!(zin && pass == 0)) {
+            c->zcmax = pass == 0 ? c->d_cmax : nullptr;  // the x pass below takes its maximum
+            const int rc = zinv<T>(c, 3, mode, 0, c->U, c->fs64, Wf(0), wfs, wp);
+            c->zcmax = nullptr;
+            H3D_TRY(rc);
+        } else {
+            H3D_CHECK(cudaMemsetAsync(c->d_cmax, 0, sizeof(unsigned long long), c->st));
+        }
         for (int s = 0; s < ns; s++)
             H3D_TRY(zinv<T>(c, 1, mode, 0, c->U + (3 + s) * c->fs64, c->fs64, Wf(6 + 3 * s), wfs, wp));
         MARK(1);
         H3D_TRY(spass<T>(c, 1, false, Wf(0), wfs, wp, 3));
         for (int s = 0; s < ns; s++) H3D_TRY(spass<T>(c, 1, false, Wf(6 + 3 * s), wfs, wp, 1));
         MARK(2);
-        if (pass == 0) H3D_CHECK(cudaMemsetAsync(c->d_cmax, 0, sizeof(unsigned long long), c->st));
         for (int s = 0; s < ns; s++) {
             FusedArgs fa;
             memset(&fa, 0, sizeof fa);
@@ -1025,13 +1034,14 @@ static int ctx_init(const hit3d_params *p, hit3d_ctx **out, double2 *ext_U, doub
     if (c->p.precision == 0) c->W64 = reinterpret_cast<double2 *>(c->W);
     else if ((rc = ctx_alloc((void **)&c->W64, f64 * 3))) { hit3d_gpu_finalize(c); return rc; }
     c->pblocks = c->nsm * 2;
+    c->nstage = c->n <= 128 ? 3 + c->nsc : 1;
     const int kpart = c->kmax + 1 > 12 ? c->kmax + 1 : 12;  // shells and the Parseval sum, or 3 fields' physical sums
     if ((rc = ctx_alloc((void **)&c->tw64, sizeof(double2) * c->n)) || (rc = ctx_alloc((void **)&c->tw32, sizeof(float2) * c->n)) ||
         (rc = ctx_alloc((void **)&c->d_fen, sizeof(double))) || (rc = ctx_alloc((void **)&c->d_cmax, 2 * sizeof(unsigned long long))) ||
         (rc = ctx_alloc((void **)&c->d_part, sizeof(double) * (size_t)c->pblocks * kpart)) ||
         (rc = ctx_alloc((void **)&c->d_red, sizeof(double) * (size_t)(c->kmax + 1 + 12))) ||
         (rc = ctx_alloc((void **)&c->d_ratio, sizeof(double) * (size_t)kpart)) ||
-        (rc = ctx_alloc((void **)&c->stage, sizeof(double2) * (size_t)c->n * c->n * c->nh))) {
+        (rc = ctx_alloc((void **)&c->stage, sizeof(double2) * (size_t)c->nstage * c->n * c->n * c->nh))) {
         hit3d_gpu_finalize(c);
         return rc;
     }
@@ -1145,6 +1155,23 @@ static int transfer_fields(hit3d_ctx *c, double2 *dev, const double *hsrc, doubl
     const size_t hp = (size_t)ld1 * sizeof(double);
     const size_t rows = (size_t)c->n * c->n;
     if (hsrc) c->alias_known = 0;
+    if (nf <= c->nstage && hp == width) {
+        // small grids: all fields with one kernel and one copy, a few microseconds
+        // each whatever the size (96 runs of 32^3 to 128^3 download 288 fields)
+        const size_t bytes = width * rows * nf;
+        const dim3 g((unsigned)std::min<int64_t>(pw_grid(c).x, ((int64_t)rows * c->nh + 255) / 256), nf);
+        if (hsrc) {
+            H3D_CHECK(cudaMemcpyAsync(c->stage, hsrc, bytes, cudaMemcpyHostToDevice, c->st));
+            k_ref_to_dev<<<g, 256, 0, c->st>>>(c->n, c->nh, c->P64, c->stage, dev, c->fs64);
+            H3D_LAUNCH_CHECK();
+        } else {
+            k_dev_to_ref<<<g, 256, 0, c->st>>>(c->n, c->nh, c->P64, dev, c->stage, c->fs64);
+            H3D_LAUNCH_CHECK();
+            H3D_CHECK(cudaMemcpyAsync(hdst, c->stage, bytes, cudaMemcpyDeviceToHost, c->st));
+        }
+        H3D_CHECK(cudaStreamSynchronize(c->st));
+        return 0;
+    }
     for (int f = 0; f < nf; f++) {
         double2 *d = dev + f * c->fs64;
         if (hsrc) {

@@ -54,6 +54,7 @@ template <typename T, typename TI, typename TO> struct IOPlain {
         return b;
     }
     H3D_D int outer(int y) const { return ko >= 0 ? kept_index(y, n, ko) : y; }
+    H3D_D void begin() const {}
     H3D_D cx<T> load(int f, int o, int c, int p) const
     {
         if (c >= ncol || (kl >= 0 && !kept(p, n, kl))) return mk<T>(0, 0);
@@ -94,6 +95,13 @@ template <typename T, typename TO, int MODE> struct IOSpec {
     int kl = -1, ko = -1;  // 2/3-rule pruning of the kz loads and the ky rows
     int nfr = 0;           // runs of a batch, as IOPlain::at
     int64_t rs_src = 0, rs_dst = 0;
+    // cleared by one thread: the Courant maximum of the x pass to come (a memset
+    // of its own is one more launch of a small grid's seven)
+    unsigned long long *zero = nullptr;
+    H3D_D void begin() const
+    {
+        if (zero != nullptr && threadIdx.x == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) *zero = 0;
+    }
     H3D_D IOSpec at(int z, int &f) const
     {
         IOSpec b = *this;
@@ -207,6 +215,7 @@ __global__ void __launch_bounds__(NT, MINB) k_colfft(const IO io, const cx<T> *_
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T> *sm = reinterpret_cast<cx<T> *>(smraw);
     using F = ColFFT<T, L, TC, NT, false, FWD, false>;
+    io.begin();
     int f;
     const IO iob = io.at(blockIdx.z, f);
     const int col0 = blockIdx.x * TC, outer = iob.outer(blockIdx.y);

@@ -1395,23 +1395,25 @@ __global__ void k_dev_to_band(int n, int kc, int pitch, const double2 *__restric
 
 // layout conversion between the reference's (nx+2, ny, nz) Fourier array
 // [ky][kz][kx] (pitch nh) and the device layout [kz][ky][kx] (pitch P)
-__global__ void k_ref_to_dev(int n, int nh, int pitch, const double2 *__restrict__ R, double2 *__restrict__ D)
+__global__ void k_ref_to_dev(int n, int nh, int pitch, const double2 *__restrict__ R, double2 *__restrict__ D, int64_t fs = 0)
 {
     const int64_t nm = (int64_t)n * n * nh;
+    R += blockIdx.y * nm;
+    D += blockIdx.y * fs;
+    const DivU64 dx(nh), dz(n);
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nm; t += (int64_t)gridDim.x * blockDim.x) {
-        int kx = (int)(t % nh);
-        int64_t r = t / nh;
-        int kzi = (int)(r % n), kyi = (int)(r / n);
-        D[((int64_t)kzi * n + kyi) * pitch + kx] = R[t];
+        const int64_t r = dx(t), kyi = dz(r), kzi = r - kyi * n;
+        D[(kzi * n + kyi) * pitch + (t - r * nh)] = R[t];
     }
 }
-__global__ void k_dev_to_ref(int n, int nh, int pitch, const double2 *__restrict__ D, double2 *__restrict__ R)
+__global__ void k_dev_to_ref(int n, int nh, int pitch, const double2 *__restrict__ D, double2 *__restrict__ R, int64_t fs = 0)
 {
     const int64_t nm = (int64_t)n * n * nh;
+    R += blockIdx.y * nm;
+    D += blockIdx.y * fs;
+    const DivU64 dx(nh), dz(n);
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nm; t += (int64_t)gridDim.x * blockDim.x) {
-        int kx = (int)(t % nh);
-        int64_t r = t / nh;
-        int kzi = (int)(r % n), kyi = (int)(r / n);
-        R[t] = D[((int64_t)kzi * n + kyi) * pitch + kx];
+        const int64_t r = dx(t), kyi = dz(r), kzi = r - kyi * n;
+        R[t] = D[(kzi * n + kyi) * pitch + (t - r * nh)];
     }
 }
