@@ -131,6 +131,7 @@ struct hit3d_ctx {
     float2 *tw32;
     double *d_fen, *d_part, *d_red, *d_ratio;
     unsigned long long *d_cmax;  // [0]: Courant maximum (bits of a double >= 0); [1]: the error word d_err
+    const double *gate;  // set while passes are issued that run only if *gate < 0 on the device
     unsigned long long *zcmax;  // set while the z pass that clears the Courant maximum is issued
     int *d_err;          // device error word: bit 1 = a fused x pass gave up waiting for its input stage
     double2 *stage;      // nstage fields in the reference layout: every state field up to 128^3, else one

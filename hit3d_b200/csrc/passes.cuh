@@ -37,6 +37,7 @@ template <typename T, typename TI, typename TO> struct IOPlain {
     int64_t sa_src, so_src, sa_dst, so_dst;
     int ncol;
     int n = 0, kl = -1, ks = -1, ko = -1;
+    const double *gate = nullptr;  // the pass is skipped unless *gate < 0
     // runs of a batch: nfr > 0 fields per run, run r's fields start rs_src /
     // rs_dst elements after run r-1's; grid index z = r * nfr + f
     int nfr = 0;
@@ -54,7 +55,7 @@ template <typename T, typename TI, typename TO> struct IOPlain {
         return b;
     }
     H3D_D int outer(int y) const { return ko >= 0 ? kept_index(y, n, ko) : y; }
-    H3D_D void begin() const {}
+    H3D_D bool begin() const { return gate == nullptr || *gate < 0.0; }
     H3D_D cx<T> load(int f, int o, int c, int p) const
     {
         if (c >= ncol || (kl >= 0 && !kept(p, n, kl))) return mk<T>(0, 0);
@@ -98,9 +99,10 @@ template <typename T, typename TO, int MODE> struct IOSpec {
     // cleared by one thread: the Courant maximum of the x pass to come (a memset
     // of its own is one more launch of a small grid's seven)
     unsigned long long *zero = nullptr;
-    H3D_D void begin() const
+    H3D_D bool begin() const
     {
         if (zero != nullptr && threadIdx.x == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) *zero = 0;
+        return true;
     }
     H3D_D IOSpec at(int z, int &f) const
     {
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(NT, MINB) k_colfft(const IO io, const cx<T> *_
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T> *sm = reinterpret_cast<cx<T> *>(smraw);
     using F = ColFFT<T, L, TC, NT, false, FWD, false>;
-    io.begin();
+    if (!io.begin()) return;
     int f;
     const IO iob = io.at(blockIdx.z, f);
     const int col0 = blockIdx.x * TC, outer = iob.outer(blockIdx.y);
@@ -335,14 +337,15 @@ __global__ void __launch_bounds__(NT) k_xc2r(cx<TS> *base, int64_t fs, int64_t p
         }
 }
 
-// plain r2c (forward x pass) of one field, in place
+// plain r2c (forward x pass) of one field, in place; gate (may be null) as IOPlain::gate
 template <typename T, int L, int TC, int NT, typename TS>
 __global__ void __launch_bounds__(NT) k_xr2c(cx<TS> *base, int64_t fs, int64_t pitch, int npairs,
-                                             const cx<T> *__restrict__ tw, int kx_lim)
+                                             const cx<T> *__restrict__ tw, int kx_lim, const double *gate)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T> *sm = reinterpret_cast<cx<T> *>(smraw);
     using F = RowFFT<T, L, TC, NT, false>;
+    if (gate != nullptr && !(*gate < 0.0)) return;
     const int pair0 = blockIdx.x * TC;
     cx<TS> *fb = base + blockIdx.z * fs;
     cx<T> in[F::NIN], out[F::NOUT];
@@ -393,6 +396,7 @@ struct FusedArgs {
     int64_t phys_fs, phys_pitch;
     double p0, p1;       // operator parameters
     int kx_lim;          // > 0: only kx < kx_lim is read and stored (2/3-rule pruning)
+    int full_phi;        // OpScal: phi is read at every kx (an LES field beyond the 2/3 rule's band)
     int *err;            // optional: set (bit 1) when a bounded wait on the input stage ran out
     int nruns;           // runs of a batch (0 or 1: one run); npairs is per run
     int64_t rstride;     // elements of cx<TS> from one run's work fields to the next run's

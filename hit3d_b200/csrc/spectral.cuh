@@ -548,20 +548,21 @@ __global__ void k_dealias_all(int n, int nh, int pitch, int64_t fs, int nf, int 
     }
 }
 
-// max |component| of nf fields of A and B over the modes the 2/3 rule removes
-// (some |k_i| > N/3), as the bit pattern of a non-negative double: zero means
-// the transforms of a time step may skip those modes exactly
-__global__ void k_alias_max(int n, int nh, int pitch, int64_t fs, int nf, const double2 *__restrict__ A,
+// max |component| of nfa fields of A and nf of B over the modes the 2/3 rule
+// removes (some |k_i| > N/3), as the bit pattern of a non-negative double: zero
+// means the transforms of a time step may skip those modes exactly
+__global__ void k_alias_max(int n, int nh, int pitch, int64_t fs, int nf, const double2 *__restrict__ A, int nfa,
                             const double2 *__restrict__ B, unsigned long long *out)
 {
     const int64_t nm = (int64_t)n * n * nh;
+    const ModeLoop ml(n, nh, -1);
     double mx = 0.0;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nm; t += (int64_t)gridDim.x * blockDim.x) {
-        ModeIdx m = mode_of(t, n, nh);
+        const ModeIdx m = ml.at(t);
         if (m.ialias > 0) {
             const int64_t o = soff(m, n, pitch);
             for (int f = 0; f < nf; f++) {
-                const double2 a = A[o + f * fs], b = B[o + f * fs];
+                const double2 a = f < nfa ? A[o + f * fs] : make_double2(0.0, 0.0), b = B[o + f * fs];
                 mx = fmax(mx, fmax(fmax(fabs(a.x), fabs(a.y)), fmax(fabs(b.x), fabs(b.y))));
             }
         }

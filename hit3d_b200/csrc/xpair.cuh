@@ -67,8 +67,9 @@ H3D_D void xp_forward(const FusedArgs &a, int o0, cx<T> (&in)[NF][ColFFT<T, L, T
 }
 
 // packed inputs of the inverse transforms from the staged rows of two fields
+// (row stride rs0, rs1 and kx limit lim0, lim1 of each)
 template <typename T, int L, int TC, int NT, typename TS>
-H3D_D void xp_load2(const FusedArgs &a, const cx<TS> *s0, const cx<TS> *s1, int rs, int pair0, int lim,
+H3D_D void xp_load2(const FusedArgs &a, const cx<TS> *s0, const cx<TS> *s1, int rs0, int rs1, int pair0, int lim0, int lim1,
                     cx<T> (&in)[2][ColFFT<T, L, TC, NT, true, false, true>::NIN])
 {
     using FI = RowFFT<T, L, TC, NT, true>;
@@ -80,8 +81,9 @@ H3D_D void xp_load2(const FusedArgs &a, const cx<TS> *s0, const cx<TS> *s1, int 
             for (int m = 0; m < FI::R0; m++) {
                 int c, p;
                 if (FI::in_slot(i, m, c, p) && pair0 + c < a.npairs) {
+                    const int rs = f == 0 ? rs0 : rs1;
                     const cx<TS> *A = (f == 0 ? s0 : s1) + 2 * c * rs;
-                    in[f][i * FI::R0 + m] = load_packed<T, L, TS>(A, A + rs, p, lim);
+                    in[f][i * FI::R0 + m] = load_packed<T, L, TS>(A, A + rs, p, f == 0 ? lim0 : lim1);
                 } else in[f][i * FI::R0 + m] = mk<T>(0, 0);
             }
 }
@@ -109,10 +111,11 @@ __global__ void __launch_bounds__(NT, MINB) k_xscal(const FusedArgs a, const cx<
     const T norm = (T)a.norm;
     const int lim = a.kx_lim > 0 ? a.kx_lim : L / 2 + 1;
     const int nch = StageRow<TS>::chunks(lim), rs = nch * StageRow<TS>::PER;
+    const int limp = a.full_phi ? L / 2 + 1 : lim, nchp = StageRow<TS>::chunks(limp), rsp = nchp * StageRow<TS>::PER;  // phi
     const int ntiles = (a.npairs + TC - 1) / TC;
     auto issue_phi_u = [&](int tile) {
         if (tile < ntiles) {
-            xp_issue<TS, 1, TC, NT>(a, 3, bp, E, tile * TC, nch);
+            xp_issue<TS, 1, TC, NT>(a, 3, bp, E, tile * TC, nchp);
             xp_issue<TS, 1, TC, NT>(a, 0, bp + E, E, tile * TC, nch);
         }
         cp_async_commit();
@@ -131,7 +134,7 @@ __global__ void __launch_bounds__(NT, MINB) k_xscal(const FusedArgs a, const cx<
         __syncthreads();
         {
             cx<T> in[2][FI::NIN], out[2][NP];
-            xp_load2<T, L, TC, NT, TS>(a, bp, bp + E, rs, pair0, lim, in);
+            xp_load2<T, L, TC, NT, TS>(a, bp, bp + E, rsp, rs, pair0, limp, lim, in);
 #pragma unroll
             for (int q = 0; q < NP; q++) out[0][q] = out[1][q] = mk<T>(0, 0);  // slots of idle butterflies
             __syncthreads();  // the staged rows are read: the buffers turn into exchange buffers
@@ -146,7 +149,7 @@ __global__ void __launch_bounds__(NT, MINB) k_xscal(const FusedArgs a, const cx<
         __syncthreads();  // v and w have arrived, the exchange buffers of phi and u are read
         {
             cx<T> in[2][FI::NIN], out[2][NP];
-            xp_load2<T, L, TC, NT, TS>(a, bv, bv + E, rs, pair0, lim, in);
+            xp_load2<T, L, TC, NT, TS>(a, bv, bv + E, rs, rs, pair0, lim, lim, in);
 #pragma unroll
             for (int q = 0; q < NP; q++) out[0][q] = out[1][q] = mk<T>(0, 0);
             __syncthreads();
@@ -204,7 +207,7 @@ __global__ void __launch_bounds__(NT, MINB) k_xsmag(const FusedArgs a, const cx<
             else if (g == 1) cp_async_wait_group<1>();
             else cp_async_wait_group<0>();
             __syncthreads();
-            xp_load2<T, L, TC, NT, TS>(a, b, b + E, rs, pair0, lim, in);
+            xp_load2<T, L, TC, NT, TS>(a, b, b + E, rs, rs, pair0, lim, lim, in);
 #pragma unroll
             for (int q = 0; q < NP; q++) out[0][q] = out[1][q] = mk<T>(0, 0);
             __syncthreads();  // the staged rows are read: the buffers turn into exchange buffers
