@@ -427,7 +427,8 @@ __global__ void k_scalar(const StepArgs a, int mode, int s, const cx<TP> *__rest
 // Bands of up to kFsmall shells: the candidate modes |k_i| <= kfmax + 1 in the
 // reference's loop order (ky, kz, kx) go in chunks of kFchunk, every thread
 // computing the contributions of its candidates (its own loads, all in flight
-// at once), and thread 0 adds them, in that order, to the shell sums.  Wider
+// at once), and thread s adds those of shell s + 1, in that order, in a register
+// (one thread with a local array of shell sums took 9 of the launch's 12 us).  Wider
 // bands: thread s of the CTA sums shell s + 1 (and s + 1 + blockDim.x, ...)
 // over the same candidates in the same order, and thread 0 adds the shells
 // (es, kfmax doubles of dynamic shared memory).  Every shell sum and the final
@@ -452,8 +453,7 @@ __global__ void k_forcing_energy(int n, int pitch, int64_t fs, int kfmax, const 
         const int nk = 2 * km + 1 < n ? 2 * km + 1 : n;
         const int nxc = (km < n / 2 - 1 ? km : n / 2 - 1) + 1;
         const int64_t nc = (int64_t)nk * nk * nxc;
-        double e16[kFsmall];
-        for (int s = 0; s < kFsmall; s++) e16[s] = 0.0;
+        double es1 = 0.0;  // threads 0..kfmax-1: the sum of shell threadIdx.x + 1
         for (int64_t base = 0; base < nc; base += kFchunk) {
             for (int q = threadIdx.x; q < kFchunk; q += blockDim.x) {
                 const int64_t t = base + q;
@@ -483,20 +483,22 @@ __global__ void k_forcing_energy(int n, int pitch, int64_t fs, int kfmax, const 
                 fsh[q] = sh8;
             }
             __syncthreads();
-            if (threadIdx.x == 0) {
+            if ((int)threadIdx.x < kfmax) {
                 const int m = nc - base < kFchunk ? (int)(nc - base) : kFchunk;
+#pragma unroll 8
                 for (int q = 0; q < m; q++) {
-                    const int sh = fsh[q];
-                    if (sh == 0) continue;
-                    e16[sh - 1] = __dadd_rn(e16[sh - 1], fr[q]);
-                    e16[sh - 1] = __dadd_rn(e16[sh - 1], fi[q]);
+                    if (fsh[q] != threadIdx.x + 1) continue;
+                    es1 = __dadd_rn(es1, fr[q]);
+                    es1 = __dadd_rn(es1, fi[q]);
                 }
             }
             __syncthreads();
         }
+        if ((int)threadIdx.x < kfmax) fr[threadIdx.x] = es1;
+        __syncthreads();
         if (threadIdx.x == 0) {
             double e = 0.0;
-            for (int s = 0; s < kfmax; s++) e = __dadd_rn(e, e16[s]);
+            for (int s = 0; s < kfmax; s++) e = __dadd_rn(e, fr[s]);
             *out = e;
         }
         return;
