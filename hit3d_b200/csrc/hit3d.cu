@@ -291,6 +291,7 @@ template <typename T> static int xr2c(hit3d_ctx *c, cx<T> *base, int64_t fs, int
 // the fused x pass (xpass.cuh), instantiated in xpass_f64.cu and xpass_f32.cu
 template <typename T, template <class> class OP> int xfused(hit3d_ctx *c, FusedArgs a);
 constexpr int kFusedVariants = HIT3D_FUSED_VARIANTS;
+constexpr int kSumBlocks = 9;  // CTAs per SM of k_xc2r_sums over its three fields
 
 static dim3 pw_grid(const hit3d_ctx *c) { return dim3(c->nsm * 4); }
 // grid of a grid-stride kernel of 256-thread CTAs that may fit fewer than four
@@ -544,8 +545,8 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
             H3D_TRY(zinv<T>(c, 1, PRE_TRUNC, 0, K, c->fs64, Wf(kf), wfs, wp));
             H3D_TRY(spass<T>(c, 1, false, Wf(kf), wfs, wp, 1));
             H3D_TRY(xc2r<T>(c, Wf(kf), wfs, wp, 1));
-            k_phys_partial<<<c->pblocks, 256, 0, c->st>>>(c->n, 2 * (int64_t)wp, 2 * wfs, 1, 2,
-                                                          reinterpret_cast<const double *>(Wf(kf)), c->d_part);
+            k_phys_partial<<<c->pblocks, 256, 0, c->st>>>(c->n, 2 * (int64_t)wp, reinterpret_cast<const double *>(Wf(kf)),
+                                                          c->d_part);
             H3D_LAUNCH_CHECK();
             k_phys_final<<<1, 32, 0, c->st>>>(c->pblocks, c->d_part, c->d_kmin);
             H3D_LAUNCH_CHECK();
@@ -1077,7 +1078,9 @@ static int ctx_init(const hit3d_params *p, hit3d_ctx **out, double2 *ext_U, doub
     else if ((rc = ctx_alloc((void **)&c->W64, f64 * 3))) { hit3d_gpu_finalize(c); return rc; }
     c->pblocks = c->nsm * 2;
     c->nstage = c->n <= 128 ? 3 + c->nsc : 1;
-    const int kpart = c->kmax + 1 > 12 ? c->kmax + 1 : 12;  // shells and the Parseval sum, or 3 fields' physical sums
+    // per statistics block (two per SM): shells and the Parseval sum, or four sums of
+    // up to kSumBlocks / 2 x-pass blocks
+    const int kpart = c->kmax + 1 > 2 * kSumBlocks ? c->kmax + 1 : 2 * kSumBlocks;
     if ((rc = ctx_alloc((void **)&c->tw64, sizeof(double2) * c->n)) || (rc = ctx_alloc((void **)&c->tw32, sizeof(float2) * c->n)) ||
         (rc = ctx_alloc((void **)&c->d_fen, sizeof(double))) || (rc = ctx_alloc((void **)&c->d_cmax, 2 * sizeof(unsigned long long))) ||
         (rc = ctx_alloc((void **)&c->d_part, sizeof(double) * (size_t)c->pblocks * kpart)) ||
@@ -1972,15 +1975,31 @@ static int shell_spectrum(hit3d_ctx *c, const double2 *src, int nf, double *es, 
     return 0;
 }
 
-// deterministic sums over physical points of nf consecutive W64 fields, each on its own
-static int phys_sums(hit3d_ctx *c, int nf, int mode)
+// deterministic sums over the physical points of nf fields, each on its own, of the
+// state with a spectral pre-operation (inv_from_state without the physical fields)
+template <int L> static int xc2r_sums_L(hit3d_ctx *c, int nf, int mode)
 {
-    k_phys_partial<<<dim3(c->pblocks, nf), 256, 0, c->st>>>(c->n, 2 * (int64_t)c->P64, 2 * c->fs64, 1, mode,
-                                                           reinterpret_cast<const double *>(c->W64), c->d_part);
+    using RC = RowCfg<double, L>;
+    const int npairs = c->n * c->n / 2;
+    auto k = k_xc2r_sums<double, L, RC::TC, RC::NT, double>;
+    H3D_TRY(set_smem(k, RC::SMEM));
+    const int tiles = (npairs + RC::TC - 1) / RC::TC;
+    const int per = kSumBlocks / 3, grid = tiles < c->nsm * per ? tiles : c->nsm * per;  // resident CTAs for 3 fields
+    const double n3 = (double)c->n * c->n * c->n;
+    k<<<dim3(grid, nf), RC::NT, RC::SMEM, c->st>>>(c->W64, c->fs64, c->P64, npairs, 1.0 / n3, c->tw64,
+                                                  c->kc_active >= 0 ? c->kc_active + 1 : 0, mode, c->d_part);
     H3D_LAUNCH_CHECK();
-    k_phys_final<<<nf, 32, 0, c->st>>>(c->pblocks, c->d_part, c->d_red + c->kmax + 1);
+    k_phys_final<<<nf, 32, 0, c->st>>>(grid, c->d_part, c->d_red + c->kmax + 1);
     H3D_LAUNCH_CHECK();
     return 0;
+}
+static int inv_sums(hit3d_ctx *c, int nf, int mode, const double2 *src, int sum_mode)
+{
+    H3D_TRY(zinv<double>(c, nf, mode, 0, src, c->fs64, c->W64, c->fs64, c->P64));
+    H3D_TRY(spass<double>(c, 1, false, c->W64, c->fs64, c->P64, nf));
+#define CALL(L) xc2r_sums_L<L>(c, nf, sum_mode)
+    H3D_DISPATCH(c->n, CALL)
+#undef CALL
 }
 // every sum of d_red: kmax + 1 + 4 nf values, in one read
 static int read_sums(hit3d_ctx *c, int nf, std::vector<double> &r)
@@ -1995,7 +2014,8 @@ static int read_sums(hit3d_ctx *c, int nf, std::vector<double> &r)
 // (Parseval, with the spectrum in one pass over the state), so that only the
 // skewness's three derivatives and a scalar's own field are transformed, with
 // the step's pruned passes when the state is zero beyond N/3.  Velocity and two
-// scalars at 256^3: 6.8 ms with a transform for every derivative, 1.08 ms now.
+// scalars at 256^3: 6.8 ms with a transform for every derivative, 0.97 ms with
+// these sums over physical fields in HBM, 0.86 ms with the sums in the x pass.
 extern "C" int hit3d_gpu_stats(hit3d_ctx *c, double *e_spec, int32_t kmax, double *o)
 {
     if (!c || !e_spec || !o) return h3d_set_error_msg(-1, "hit3d_gpu_stats: null argument");
@@ -2010,8 +2030,7 @@ extern "C" int hit3d_gpu_stats(hit3d_ctx *c, double *e_spec, int32_t kmax, doubl
         // spectrum and enstrophy (m_stats.f90:99-189, 241-289)
         H3D_TRY(shell_sums(c, c->U, 3, 0.5, SPEC_CURL, c->kc_active));
         // skewness of the longitudinal derivatives
-        H3D_TRY(inv_from_state(c, 3, PRE_DLONG, 0, c->U));
-        H3D_TRY(phys_sums(c, 3, 1));
+        H3D_TRY(inv_sums(c, 3, PRE_DLONG, c->U, 1));
     }
     H3D_TRY(read_sums(c, 3, r));
     memcpy(e_spec, r.data(), sizeof(double) * kmax);
@@ -2058,8 +2077,7 @@ extern "C" int hit3d_gpu_scalar_stats(hit3d_ctx *c, int32_t s, double *spec, int
         PruneScope prune_scope(c);
         if (s >= c->p.n_scalars) c->kc_active = -1;  // an LES field may lie beyond N/3
         H3D_TRY(shell_sums(c, phi, 1, 0.5, SPEC_GRAD, c->kc_active));
-        H3D_TRY(inv_from_state(c, 1, PRE_COPY, 0, phi));
-        H3D_TRY(phys_sums(c, 1, 2));
+        H3D_TRY(inv_sums(c, 1, PRE_COPY, phi, 2));
     }
     H3D_TRY(read_sums(c, 1, r));
     for (int k = 0; k < kmax; k++) spec[k] = 2.0 * r[k];

@@ -337,6 +337,73 @@ __global__ void __launch_bounds__(NT) k_xc2r(cx<TS> *base, int64_t fs, int64_t p
         }
 }
 
+// Sums over the physical points of the fields (blockIdx.y) without the physical
+// fields reaching HBM: the inverse x pass with a reduction in place of its stores,
+// part[field][block][4] as k_phys_partial's.  mode 1: x^2 and x^3; mode 2: x, x^2,
+// min, max.  A grid of resident CTAs walks the row pairs, each thread adds its
+// points in a fixed order.
+template <typename T, int L, int TC, int NT, typename TS>
+__global__ void __launch_bounds__(NT) k_xc2r_sums(const cx<TS> *base, int64_t fs, int64_t pitch, int npairs, T norm,
+                                                  const cx<T> *__restrict__ tw, int kx_lim, int mode, double *__restrict__ part)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ double sh[4][NT / 32];
+    cx<T> *sm = reinterpret_cast<cx<T> *>(smraw);
+    using F = RowFFT<T, L, TC, NT, true>;
+    const cx<TS> *fb = base + blockIdx.y * fs;
+    const int lim = kx_lim > 0 ? kx_lim : L / 2 + 1;
+    double s0 = 0.0, s1 = 0.0, mn = 1e300, mx = -1e300;
+#pragma unroll 1
+    for (int pair0 = blockIdx.x * TC; pair0 < npairs; pair0 += gridDim.x * TC) {
+        cx<T> in[F::NIN], out[F::NOUT];
+#pragma unroll
+        for (int i = 0; i < F::NB0; i++)
+#pragma unroll
+            for (int m = 0; m < F::R0; m++) {
+                int c, p;
+                if (F::in_slot(i, m, c, p) && pair0 + c < npairs) {
+                    const cx<TS> *A = fb + (int64_t)(2 * (pair0 + c)) * pitch;
+                    in[i * F::R0 + m] = load_packed<T, L, TS>(A, A + pitch, p, lim);
+                } else in[i * F::R0 + m] = mk<T>(0, 0);
+            }
+        F::run(in, sm, out, tw);
+        __syncthreads();  // the exchange buffer is read
+#pragma unroll
+        for (int i = 0; i < F::NBL; i++)
+#pragma unroll
+            for (int m = 0; m < F::RL; m++) {
+                int c, p;
+                if (F::out_slot(i, m, c, p) && pair0 + c < npairs) {
+                    const double a = (double)(out[i * F::RL + m].x * norm), b = (double)(out[i * F::RL + m].y * norm);
+                    if (mode == 1) {
+                        s0 += a * a + b * b;
+                        s1 += a * a * a + b * b * b;
+                    } else {
+                        s0 += a + b;
+                        s1 += a * a + b * b;
+                        mn = fmin(mn, fmin(a, b));
+                        mx = fmax(mx, fmax(a, b));
+                    }
+                }
+            }
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+        s0 += __shfl_xor_sync(0xffffffffu, s0, off);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, off);
+        mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    }
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) { sh[0][w] = s0; sh[1][w] = s1; sh[2][w] = mn; sh[3][w] = mx; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double a0 = 0.0, a1 = 0.0, a2 = 1e300, a3 = -1e300;
+        for (int i = 0; i < NT / 32; i++) { a0 += sh[0][i]; a1 += sh[1][i]; a2 = fmin(a2, sh[2][i]); a3 = fmax(a3, sh[3][i]); }
+        double *o = part + 4 * ((int64_t)blockIdx.y * gridDim.x + blockIdx.x);
+        o[0] = a0; o[1] = a1; o[2] = a2; o[3] = a3;
+    }
+}
+
 // plain r2c (forward x pass) of one field, in place; gate (may be null) as IOPlain::gate
 template <typename T, int L, int TC, int NT, typename TS>
 __global__ void __launch_bounds__(NT) k_xr2c(cx<TS> *base, int64_t fs, int64_t pitch, int npairs,

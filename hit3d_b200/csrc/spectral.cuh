@@ -750,42 +750,26 @@ __global__ void k_shell_final(int nblk, int kmax, const double *__restrict__ par
     if (lane == 0) out[s] = acc;
 }
 
-// Deterministic sums over physical points of the fields:
-// mode 0: sum_f x_f^2;  mode 1: x_0^2 and x_0^3 (two sums);  mode 2: x, x^2, min, max of x_0
-// of the field (or first of nf fields) at X + blockIdx.y fs.  A warp walks whole
-// rows, 16 bytes a lane (rows start on 16 bytes: the pitch is even), with no
-// division per point: one field of 256^3 takes 0.024 ms (134 MB), where a 64-bit
-// division per point took 0.15.
-__global__ void __launch_bounds__(256) k_phys_partial(int n, int64_t rpitch, int64_t fs, int nf, int mode,
-                                                      const double *__restrict__ X,
-                                                      double *__restrict__ part /* [gridDim.y][gridDim.x][4] */)
+// Deterministic sums over the physical points of one field: x, x^2, min, max into
+// part[block][4].  A warp walks whole rows, 16 bytes a lane (rows start on 16
+// bytes: the pitch is even), with no division per point: one field of 256^3 takes
+// 0.024 ms (134 MB), where a 64-bit division per point took 0.15.
+__global__ void __launch_bounds__(256) k_phys_partial(int n, int64_t rpitch, const double *__restrict__ X,
+                                                      double *__restrict__ part /* [gridDim.x][4] */)
 {
     __shared__ double sh[4][8];
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int rows = n * n, nv = n / 2;
-    X += blockIdx.y * fs;
     double s0 = 0.0, s1 = 0.0, mn = 1e300, mx = -1e300;
     for (int row = blockIdx.x * nw + w; row < rows; row += gridDim.x * nw) {
-        const double *p = X + row * rpitch;
+        const double2 *p = reinterpret_cast<const double2 *>(X + row * rpitch);
 #pragma unroll 4
         for (int x = l; x < nv; x += 32) {
-            const double2 v = reinterpret_cast<const double2 *>(p)[x];
-            if (mode == 0) {
-                double2 q = make_double2(v.x * v.x, v.y * v.y);
-                for (int f = 1; f < nf; f++) {
-                    const double2 u = reinterpret_cast<const double2 *>(p + f * fs)[x];
-                    q = make_double2(q.x + u.x * u.x, q.y + u.y * u.y);
-                }
-                s0 += q.x + q.y;
-            } else if (mode == 1) {
-                s0 += v.x * v.x + v.y * v.y;
-                s1 += v.x * v.x * v.x + v.y * v.y * v.y;
-            } else {
-                s0 += v.x + v.y;
-                s1 += v.x * v.x + v.y * v.y;
-                mn = fmin(mn, fmin(v.x, v.y));
-                mx = fmax(mx, fmax(v.x, v.y));
-            }
+            const double2 v = p[x];
+            s0 += v.x + v.y;
+            s1 += v.x * v.x + v.y * v.y;
+            mn = fmin(mn, fmin(v.x, v.y));
+            mx = fmax(mx, fmax(v.x, v.y));
         }
     }
     for (int off = 16; off > 0; off >>= 1) {
@@ -799,7 +783,7 @@ __global__ void __launch_bounds__(256) k_phys_partial(int n, int64_t rpitch, int
     if (threadIdx.x == 0) {
         double a0 = 0.0, a1 = 0.0, a2 = 1e300, a3 = -1e300;
         for (int i = 0; i < nw; i++) { a0 += sh[0][i]; a1 += sh[1][i]; a2 = fmin(a2, sh[2][i]); a3 = fmax(a3, sh[3][i]); }
-        double *o = part + 4 * ((int64_t)blockIdx.y * gridDim.x + blockIdx.x);
+        double *o = part + 4 * (int64_t)blockIdx.x;
         o[0] = a0; o[1] = a1; o[2] = a2; o[3] = a3;
     }
 }
