@@ -143,6 +143,8 @@ static int zinv_L(hit3d_ctx *c, int nf, int mode, int sfield, const double2 *src
     if constexpr (std::is_same<T, double>::value) {
         // statistics pre-operations run in FP64 only
         switch (mode) {
+        case PRE_STRAIN_Z: return zinv_LM<T, L, PRE_STRAIN_Z>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
+        case PRE_GRAD_Z: return zinv_LM<T, L, PRE_GRAD_Z>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
         case PRE_CURL: return zinv_LM<T, L, PRE_CURL>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
         case PRE_DLONG: return zinv_LM<T, L, PRE_DLONG>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
         case PRE_TRUNC: return zinv_LM<T, L, PRE_TRUNC>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
@@ -158,6 +160,32 @@ static int zinv(hit3d_ctx *c, int nf, int mode, int sfield, const double2 *src, 
                 int64_t dst_fs, int dpitch)
 {
 #define CALL(L) zinv_L<T, L>(c, nf, mode, sfield, src, src_fs, dst, dst_fs, dpitch)
+    H3D_DISPATCH(c->n, CALL)
+#undef CALL
+}
+
+// z and y inverse of the velocity's strains (six fields d) or gradients (nine), given
+// the velocity's own z inverse in w (IODeriv)
+template <int L, bool GRAD> static int deriv_inv_L(hit3d_ctx *c, const double2 *w, double2 *d, int64_t fs, int pitch)
+{
+    H3D_TRY((zinv_L<double, L>(c, 3, GRAD ? PRE_GRAD_Z : PRE_STRAIN_Z, 0, c->U, c->fs64, d, fs, pitch)));
+    using CF = ColCfgT<double, L, true, 0>;
+    IODeriv<GRAD> io;
+    io.w = w; io.d = d; io.fs = fs; io.sa = pitch; io.so = (int64_t)c->n * pitch;
+    io.n = c->n; io.ncol = c->nh;
+    if (c->kc_active >= 0) {
+        io.kl = c->kc_active;
+        io.ncol = c->kc_active + 1;
+    }
+    auto k = k_colfft<double, L, CF::TC, CF::NT, false, IODeriv<GRAD>, CF::MINB>;
+    H3D_TRY(set_smem(k, CF::SMEM));
+    k<<<dim3((io.ncol + CF::TC - 1) / CF::TC, c->n, GRAD ? 9 : 6), CF::NT, CF::SMEM, c->st>>>(io, twid<double>(c));
+    H3D_LAUNCH_CHECK();
+    return 0;
+}
+template <bool GRAD> static int deriv_inv(hit3d_ctx *c, const double2 *w, double2 *d, int64_t fs, int pitch)
+{
+#define CALL(L) deriv_inv_L<L, GRAD>(c, w, d, fs, pitch)
     H3D_DISPATCH(c->n, CALL)
 #undef CALL
 }
@@ -533,6 +561,9 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
     const int nps = p.n_scalars, kf0 = 3 + p.n_scalars;  // kf0: first LES field of the state
     const int kf = nprod + (lag ? 18 : 10) + 3 * nps, nutf = kf + 1;
 
+    // FP64: the velocity's derivatives are made beside its own inverse (deriv_inv)
+    const bool deriv = std::is_same<T, double>::value && (les || les_mlp || dlm);
+
     MARK(7);
     if constexpr (std::is_same<T, double>::value) {
         if (dlm) {
@@ -615,6 +646,15 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
         };
         for (int s = 0; s < ns; s++)
             H3D_TRY(field_pass(s, [&] { return zinv<T>(c, 1, mode, 0, c->U + (3 + s) * c->fs64, c->fs64, Wf(6 + 3 * s), wfs, wp); }));
+        if constexpr (std::is_same<T, double>::value) {
+            // while the velocity's z inverse is there: strains or gradients of the
+            // closures below, as far as their x pass
+            if (deriv) {
+                MARK(6);
+                if (les_mlp) H3D_TRY(deriv_inv<true>(c, Wf(0), Wf(nprod), wfs, wp));
+                else H3D_TRY(deriv_inv<false>(c, Wf(0), Wf(nprod), wfs, wp));
+            }
+        }
         MARK(1);
         H3D_TRY(spass<T>(c, 1, false, Wf(0), wfs, wp, 3));
         for (int s = 0; s < ns; s++)
@@ -684,12 +724,14 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
             // Smagorinsky with passive scalars: stress and the scalars' turbulent
             // fluxes nu_t grad(phi) from the physical fields (m_les.f90:1142-1215,
             // 902-1018, 1028-1091)
-            const int t0 = nprod, nf = 6 + 3 * ns;
-            H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_A, 0, c->U, c->fs64, Wf(t0), wfs, wp));
-            H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_B, 0, c->U, c->fs64, Wf(t0 + 3), wfs, wp));
+            const int t0 = nprod, nf = 6 + 3 * ns, y0 = deriv ? 6 : 0;
+            if (!deriv) {
+                H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_A, 0, c->U, c->fs64, Wf(t0), wfs, wp));
+                H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_B, 0, c->U, c->fs64, Wf(t0 + 3), wfs, wp));
+            }
             for (int s = 0; s < ns; s++)
                 H3D_TRY(zinv<T>(c, 3, PRE_GRAD, 3 + s, c->U, c->fs64, Wf(t0 + 6 + 3 * s), wfs, wp));
-            H3D_TRY(spass<T>(c, 1, false, Wf(t0), wfs, wp, nf));
+            H3D_TRY(spass<T>(c, 1, false, Wf(t0 + y0), wfs, wp, nf - y0));
             H3D_TRY(xc2r<T>(c, Wf(t0), wfs, wp, nf));
             const double cd = p.c_smag * c->dx;
             k_smag_phys<T><<<pw_grid(c), 256, 0, c->st>>>(c->n, 2 * (int64_t)wp, 2 * wfs, cd * cd,
@@ -704,9 +746,11 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
             MARK(6);
             // Smagorinsky stress from the same state (m_les.f90:1142-1215, 902-1018)
             const int t0 = nprod;
-            H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_A, 0, c->U, c->fs64, Wf(t0), wfs, wp));
-            H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_B, 0, c->U, c->fs64, Wf(t0 + 3), wfs, wp));
-            H3D_TRY(spass<T>(c, 1, false, Wf(t0), wfs, wp, 6));
+            if (!deriv) {
+                H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_A, 0, c->U, c->fs64, Wf(t0), wfs, wp));
+                H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_B, 0, c->U, c->fs64, Wf(t0 + 3), wfs, wp));
+                H3D_TRY(spass<T>(c, 1, false, Wf(t0), wfs, wp, 6));
+            }
             FusedArgs fa;
             memset(&fa, 0, sizeof fa);
             for (int f = 0; f < 6; f++) { fa.in[f] = Wf(t0 + f); fa.out[f] = Wf(t0 + f); }
@@ -802,15 +846,13 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
                 // (les_model 3; m_les.f90:720-724, 1422-1561, 1629-1684, 1041-1091)
                 MARK(6);
                 const int t0 = nprod;
-                H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_A, 0, c->U, c->fs64, Wf(t0), wfs, wp));
-                H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_B, 0, c->U, c->fs64, Wf(t0 + 3), wfs, wp));
                 const int ninv = 17 + 3 * nps;
                 H3D_TRY(zinv<T>(c, 2, PRE_COPY, 0, c->U + (kf0 + 1) * c->fs64, c->fs64, Wf(t0 + 6), wfs, wp));
                 for (int j = 0; j < 3; j++)
                     H3D_TRY(zinv<T>(c, 3, PRE_GRAD, kf0 + j, c->U, c->fs64, Wf(t0 + 8 + 3 * j), wfs, wp));
                 for (int s = 0; s < nps; s++)
                     H3D_TRY(zinv<T>(c, 3, PRE_GRAD, 3 + s, c->U, c->fs64, Wf(t0 + 17 + 3 * s), wfs, wp));
-                H3D_TRY(spass<T>(c, 1, false, Wf(t0), wfs, wp, ninv));
+                H3D_TRY(spass<T>(c, 1, false, Wf(t0 + 6), wfs, wp, ninv - 6));
                 H3D_TRY(xc2r<T>(c, Wf(t0), wfs, wp, ninv));
                 k_dll_phys<<<pw_grid(c), 256, 0, c->st>>>(
                     c->n, 2 * (int64_t)wp, 2 * wfs, c->dx, 1.0, reinterpret_cast<const double *>(Wf(nutf)),
@@ -832,13 +874,11 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
                 // 1422-1621, 1041-1091), all from the physical fields of this state
                 MARK(6);
                 const int t0 = nprod;
-                H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_A, 0, c->U, c->fs64, Wf(t0), wfs, wp));
-                H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_B, 0, c->U, c->fs64, Wf(t0 + 3), wfs, wp));
                 const int nall = 10 + 3 * nps;
                 H3D_TRY(zinv<T>(c, 1, PRE_CUBE, 0, c->U + kf0 * c->fs64, c->fs64, Wf(t0 + 6), wfs, wp));
                 for (int s = 0; s < nps; s++)
                     H3D_TRY(zinv<T>(c, 3, PRE_GRAD, 3 + s, c->U, c->fs64, Wf(t0 + 10 + 3 * s), wfs, wp));
-                H3D_TRY(spass<T>(c, 1, false, Wf(t0), wfs, wp, 7));
+                H3D_TRY(spass<T>(c, 1, false, Wf(t0 + 6), wfs, wp, 1));
                 H3D_TRY(xc2r<T>(c, Wf(t0), wfs, wp, 7));
                 if (nps > 0) {
                     H3D_TRY(spass<T>(c, 1, false, Wf(t0 + 10), wfs, wp, 3 * nps));
@@ -871,8 +911,10 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
             // learned closure: the nine velocity gradients in physical space, the
             // network per point, the six stresses back to spectral space
             const int t0 = nprod;
-            for (int i = 0; i < 3; i++) H3D_TRY(zinv<T>(c, 3, PRE_GRAD, i, c->U, c->fs64, Wf(t0 + 3 * i), wfs, wp));
-            H3D_TRY(spass<T>(c, 1, false, Wf(t0), wfs, wp, 9));
+            if (!deriv) {
+                for (int i = 0; i < 3; i++) H3D_TRY(zinv<T>(c, 3, PRE_GRAD, i, c->U, c->fs64, Wf(t0 + 3 * i), wfs, wp));
+                H3D_TRY(spass<T>(c, 1, false, Wf(t0), wfs, wp, 9));
+            }
             H3D_TRY(xc2r<T>(c, Wf(t0), wfs, wp, 9));
             H3D_TRY(h3d_mlp_apply(c->st, sizeof(T) == 8, (int64_t)c->n * c->n * c->n, c->n, 2 * (int64_t)wp, 2 * wfs,
                                   c->mlp_delta, c->mlp_clip, c->mlp_kernel, c->mlp_wb, Wf(t0), c->d_mlp_err));
