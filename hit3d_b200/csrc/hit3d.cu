@@ -660,7 +660,23 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
         for (int s = 0; s < ns; s++)
             H3D_TRY(field_pass(s, [&] { return spass<T>(c, 1, false, Wf(6 + 3 * s), wfs, wp, 1); }));
         MARK(2);
-        for (int s = 0; s < ns; s++) {
+        int s0 = 0;
+        if constexpr (std::is_same<T, double>::value) {
+            // passive scalars two at a time
+            for (; c->n <= kScalPairMaxN && s0 + 1 < (ns < nps ? ns : nps); s0 += 2) {
+                FusedArgs fa;
+                memset(&fa, 0, sizeof fa);
+                for (int f = 0; f < 3; f++) fa.in[f] = Wf(f);
+                for (int f = 0; f < 2; f++) {
+                    fa.in[3 + f] = Wf(6 + 3 * (s0 + f));
+                    for (int o = 0; o < 3; o++) fa.out[2 * o + f] = Wf(6 + 3 * (s0 + f) + o);
+                }
+                fa.pitch = wp;
+                fa.err = c->d_err;
+                H3D_TRY((xfused<T, OpScal2>(c, fa)));
+            }
+        }
+        for (int s = s0; s < ns; s++) {
             FusedArgs fa;
             memset(&fa, 0, sizeof fa);
             fa.in[0] = Wf(0); fa.in[1] = Wf(1); fa.in[2] = Wf(2); fa.in[3] = Wf(6 + 3 * s);

@@ -28,6 +28,11 @@ template <typename T, int L> struct RowCfg {
     static constexpr size_t SMEM = (size_t)Lay<L, TC, true>::elems * sizeof(cx<T>);
 };
 
+// largest grid whose passive scalars share an x pass two at a time (k_xscal2): a
+// longer row spills its registers (512^3: both scalars' and the velocity's x pass
+// 10.1 ms paired, 9.97 one by one; 256^3 1.08 against 1.26)
+constexpr int kScalPairMaxN = 256;
+
 // Column-tile shapes the tuners pick from (ct = the context's `ctile`): 0 the
 // default ColCfg, 1 half as many kx columns per CTA, 2 twice as many (grids up
 // to 512; at least one warp per CTA), 3 the pipelined pass (k_colfft_pipe,

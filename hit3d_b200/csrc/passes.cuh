@@ -1127,6 +1127,12 @@ template <typename T> struct OpScal {
     H3D_D T out(int o, const T *v, T) const { return v[3] * v[o]; }
 };
 
+// two scalars: u v w phi psi -> phi u, psi u, phi v, psi v, phi w, psi w
+// (xpair.cuh: FP64)
+template <typename T> struct OpScal2 {
+    static constexpr int NIN = 5, NOUT = 6;
+};
+
 // Smagorinsky: inputs S11 S12 S13 S22 S23 S33, aux = nu_t = (Cs Delta)^2 sqrt(2 S:S)
 // (m_les.f90:1176-1212), outputs tau_ij = -2 nu_t S_ij (m_les.f90:935,989).
 // p0 = (Cs Delta)^2

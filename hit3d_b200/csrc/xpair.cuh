@@ -88,6 +88,26 @@ H3D_D void xp_load2(const FusedArgs &a, const cx<TS> *s0, const cx<TS> *s1, int 
             }
 }
 
+// the same of NF fields staged E elements apart
+template <typename T, int L, int TC, int NT, int NF, typename TS>
+H3D_D void xp_load(const FusedArgs &a, const cx<TS> *s, int E, int rs, int pair0, int lim,
+                   cx<T> (&in)[NF][ColFFT<T, L, TC, NT, true, false, true>::NIN])
+{
+    using FI = RowFFT<T, L, TC, NT, true>;
+#pragma unroll
+    for (int f = 0; f < NF; f++)
+#pragma unroll
+        for (int i = 0; i < FI::NB0; i++)
+#pragma unroll
+            for (int m = 0; m < FI::R0; m++) {
+                int c, p;
+                if (FI::in_slot(i, m, c, p) && pair0 + c < a.npairs) {
+                    const cx<TS> *A = s + f * E + 2 * c * rs;
+                    in[f][i * FI::R0 + m] = load_packed<T, L, TS>(A, A + rs, p, lim);
+                } else in[f][i * FI::R0 + m] = mk<T>(0, 0);
+            }
+}
+
 // Scalar fluxes.  Inputs u, v, w, phi (a.in[0..4)), outputs phi u, phi v, phi w.
 // phi and u are inverse-transformed together, then v and w with phi and phi u
 // waiting in registers; the three products go forward in lockstep.  Five buffers,
@@ -163,6 +183,100 @@ __global__ void __launch_bounds__(NT, MINB) k_xscal(const FusedArgs a, const cx<
         }
         __syncthreads();  // the exchange buffers are read
         xp_forward<T, L, TC, NT, 3, TS>(a, 0, prod, sm, tw, pair0, lim);
+        issue_v_w(tile + (int)gridDim.x);
+    }
+    cp_async_wait_all();
+}
+
+// Scalar fluxes of two scalars.  Inputs u, v, w, phi, psi (a.in[0..5)), outputs
+// phi u, psi u, phi v, psi v, phi w, psi w.  The velocity's three inverse transforms
+// serve both scalars (11 transforms in five steps, where two passes of k_xscal take
+// 14 in six).  phi, psi and u go back together, phi and psi stay in registers, the
+// products leave two at a time.  Five buffers as k_xscal's: phi, psi and u in 0, 1
+// and 2 while the rows of v and w wait in 3 and 4, and the other way round.
+// Velocity and two scalars' x passes of a step, FP64 pruned: 128^3 0.173 -> 0.158 ms,
+// 256^3 1.26 -> 1.08 ms.
+template <typename T, int L, int TC, int NT, typename TS, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_xscal2(const FusedArgs a, const cx<T> *__restrict__ tw)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    using FI = RowFFT<T, L, TC, NT, true>;
+    using FF = RowFFT<T, L, TC, NT, false>;
+    static_assert(FI::NOUT == FF::NIN && sizeof(T) == sizeof(TS), "slot hand-off mismatch");
+    constexpr int NP = FI::NOUT, E = Lay<L, TC, true>::elems;
+    static_assert(2 * StageRow<TS>::chunks(L / 2 + 1) * StageRow<TS>::PER <= L + L / 8 && E * sizeof(cx<T>) % 16 == 0, "stage");
+    cx<T> *sm = reinterpret_cast<cx<T> *>(smraw);
+    cx<T> *bv = sm + 3 * E;  // v and w
+    const T norm = (T)a.norm;
+    const int lim = a.kx_lim > 0 ? a.kx_lim : L / 2 + 1;
+    const int nch = StageRow<TS>::chunks(lim), rs = nch * StageRow<TS>::PER;
+    const int ntiles = (a.npairs + TC - 1) / TC;
+    auto issue_scal_u = [&](int tile) {
+        if (tile < ntiles) {
+            xp_issue<TS, 2, TC, NT>(a, 3, sm, E, tile * TC, nch);
+            xp_issue<TS, 1, TC, NT>(a, 0, sm + 2 * E, E, tile * TC, nch);
+        }
+        cp_async_commit();
+    };
+    auto issue_v_w = [&](int tile) {
+        if (tile < ntiles) xp_issue<TS, 2, TC, NT>(a, 1, bv, E, tile * TC, nch);
+        cp_async_commit();
+    };
+    issue_scal_u(blockIdx.x);
+    issue_v_w(blockIdx.x);
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int pair0 = tile * TC;
+        cx<T> phi[NP], psi[NP];
+        cp_async_wait_group<1>();
+        __syncthreads();
+        {
+            cx<T> prod[2][NP];
+            {
+                cx<T> in[3][FI::NIN], out[3][NP];
+                xp_load<T, L, TC, NT, 3, TS>(a, sm, E, rs, pair0, lim, in);
+#pragma unroll
+                for (int q = 0; q < NP; q++) out[0][q] = out[1][q] = out[2][q] = mk<T>(0, 0);  // slots of idle butterflies
+                __syncthreads();  // the staged rows are read: the buffers turn into exchange buffers
+                FI::template run_multi<3>(in, sm, out, tw);
+#pragma unroll
+                for (int q = 0; q < NP; q++) {
+                    const cx<T> u = mk<T>(out[2][q].x * norm, out[2][q].y * norm);
+                    phi[q] = mk<T>(out[0][q].x * norm, out[0][q].y * norm);
+                    psi[q] = mk<T>(out[1][q].x * norm, out[1][q].y * norm);
+                    prod[0][q] = mk<T>(phi[q].x * u.x, phi[q].y * u.y);
+                    prod[1][q] = mk<T>(psi[q].x * u.x, psi[q].y * u.y);
+                }
+            }
+            __syncthreads();  // the exchange buffers are read
+            xp_forward<T, L, TC, NT, 2, TS>(a, 0, prod, sm, tw, pair0, lim);
+        }
+        cp_async_wait_group<0>();
+        __syncthreads();  // v and w have arrived
+        {
+            cx<T> pv[2][NP], pw[2][NP];
+            {
+                cx<T> in[2][FI::NIN], out[2][NP];
+                xp_load<T, L, TC, NT, 2, TS>(a, bv, E, rs, pair0, lim, in);
+#pragma unroll
+                for (int q = 0; q < NP; q++) out[0][q] = out[1][q] = mk<T>(0, 0);
+                __syncthreads();
+                issue_scal_u(tile + (int)gridDim.x);
+                FI::template run_multi<2>(in, bv, out, tw);
+#pragma unroll
+                for (int q = 0; q < NP; q++) {
+                    const cx<T> v = mk<T>(out[0][q].x * norm, out[0][q].y * norm);
+                    const cx<T> w = mk<T>(out[1][q].x * norm, out[1][q].y * norm);
+                    pv[0][q] = mk<T>(phi[q].x * v.x, phi[q].y * v.y);
+                    pv[1][q] = mk<T>(psi[q].x * v.x, psi[q].y * v.y);
+                    pw[0][q] = mk<T>(phi[q].x * w.x, phi[q].y * w.y);
+                    pw[1][q] = mk<T>(psi[q].x * w.x, psi[q].y * w.y);
+                }
+            }
+            __syncthreads();
+            xp_forward<T, L, TC, NT, 2, TS>(a, 2, pv, bv, tw, pair0, lim);
+            xp_forward<T, L, TC, NT, 2, TS>(a, 4, pw, bv, tw, pair0, lim);
+        }
         issue_v_w(tile + (int)gridDim.x);
     }
     cp_async_wait_all();

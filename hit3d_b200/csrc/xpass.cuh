@@ -152,7 +152,7 @@ template <typename T, template <class> class OP, int L> static int xpair_L(hit3d
 {
     using RC = RowCfgSmall<T, L>;
     constexpr int NIN = OP<T>::NIN, MINB = RC::MINB;
-    static_assert(NIN == 4 || NIN == 6, "scalar fluxes or Smagorinsky stress");
+    static_assert(NIN >= 4 && NIN <= 6, "scalar fluxes or Smagorinsky stress");
     for (int f = 0; f < NIN; f++)
         if (reinterpret_cast<uintptr_t>(a.in[f]) % 16 != 0)
             return h3d_set_error_msg(-1, "fused x pass: input field not 16-byte aligned");
@@ -173,7 +173,9 @@ template <typename T, template <class> class OP, int L> static int xpair_L(hit3d
         return 0;
     };
     if constexpr (NIN == 4) return go(k_xscal<T, L, RC::TC, RC::NT, T, MINB>, 5 * RC::SMEM);
-    else return go(k_xsmag<T, L, RC::TC, RC::NT, T, MINB>, 6 * RC::SMEM);
+    else if constexpr (NIN == 6) return go(k_xsmag<T, L, RC::TC, RC::NT, T, MINB>, 6 * RC::SMEM);
+    else if constexpr (L <= kScalPairMaxN) return go(k_xscal2<T, L, RC::TC, RC::NT, T, MINB>, 5 * RC::SMEM);
+    else return h3d_set_error_msg(-1, "fused x pass: no paired scalars at this size");
 }
 
 template <typename T, template <class> class OP, int L> static int xfused_L(hit3d_ctx *c, FusedArgs a)
