@@ -190,7 +190,9 @@ int hit3d_gpu_set_variant(hit3d_ctx *ctx, int32_t variant);
  * that are zero or that the update masks (rhs_velocity.f90:85-142).  The
  * result is bit-identical; the state is checked on the device before the
  * first step after every change, and a state with energy beyond N/3 runs the
- * full transforms.  hit3d_gpu_pruned returns 1 if the next step is pruned. */
+ * full transforms.  With les_model 2 everything but k_sgs is pruned (clipping
+ * brings k_sgs modes beyond N/3).  hit3d_gpu_pruned returns 1 if the next step
+ * is pruned. */
 int hit3d_gpu_set_pruning(hit3d_ctx *ctx, int32_t on);
 int hit3d_gpu_pruned(hit3d_ctx *ctx);
 
@@ -282,8 +284,8 @@ int hit3d_gpu_xfft3d(hit3d_ctx *ctx, int32_t flag, const double *in, double *out
  * counterpart in the reference.  `in` is a physical (nx+2, ny, nz) device array,
  * `out` receives the Fourier (nx+2, ny, nz) array; both belong to the caller
  * and must be 16-byte aligned.  They may be the same buffer (an in-place
- * transform) or overlap: the whole input is copied into the scratch array before
- * anything is written to `out`.  Work is queued on `stream` (a cudaStream_t,
+ * transform) or overlap: the whole input has gone through its first transforms
+ * into the scratch array before anything is written to `out`.  Work is queued on `stream` (a cudaStream_t,
  * NULL = default stream) and the caller synchronises.  Grid sizes 32, 48, 64 and
  * 128 only: the one scratch field lives in a file-scope __device__ array (17 MB,
  * held on every GPU that loads the library until the process exits).  The first
