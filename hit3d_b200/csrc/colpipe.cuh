@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(NT, MINB) k_colfft_pipe(const IO io, const cx<
     };
 
     const int t0 = blockIdx.x;
-    if (!io.begin()) return;
+    if (!io.template begin<L>()) return;
     issue(t0, 0);
     issue(t0 + (int)gridDim.x, 1);
     int b = 0;

@@ -196,7 +196,6 @@ static int spass_LAC(hit3d_ctx *c, int axis, bool fwd, cx<T> *base, int64_t fs, 
 {
     using CF = ColCfgT<T, L, YPASS, CT>;
     IOPlain<T, T, T> io;
-    io.gate = c->gate;
     io.src = base; io.dst = base; io.fs_src = fs; io.fs_dst = fs; io.ncol = c->nh;
     if (axis == 1) { io.sa_src = io.sa_dst = pitch; io.so_src = io.so_dst = (int64_t)c->n * pitch; }
     else { io.sa_src = io.sa_dst = (int64_t)c->n * pitch; io.so_src = io.so_dst = pitch; }
@@ -232,13 +231,29 @@ static int spass_LAC(hit3d_ctx *c, int axis, bool fwd, cx<T> *base, int64_t fs, 
     H3D_LAUNCH_CHECK();
     return 0;
 }
+// the unpruned forward pass of one run, skipped on the device unless *c->gate < 0
+template <int L, bool YPASS> static int spass_gated_L(hit3d_ctx *c, int axis, double2 *base, int64_t fs, int pitch, int nf)
+{
+    using CF = ColCfgT<double, L, YPASS, 0>;
+    IOGated<double> io;
+    io.gate = c->gate;
+    io.src = base; io.dst = base; io.fs_src = fs; io.fs_dst = fs; io.ncol = c->nh;
+    if (axis == 1) { io.sa_src = io.sa_dst = pitch; io.so_src = io.so_dst = (int64_t)c->n * pitch; }
+    else { io.sa_src = io.sa_dst = (int64_t)c->n * pitch; io.so_src = io.so_dst = pitch; }
+    auto k = k_colfft<double, L, CF::TC, CF::NT, true, IOGated<double>, CF::MINB>;
+    H3D_TRY(set_smem(k, CF::SMEM));
+    k<<<dim3((io.ncol + CF::TC - 1) / CF::TC, c->n, nf), CF::NT, CF::SMEM, c->st>>>(io, twid<double>(c));
+    H3D_LAUNCH_CHECK();
+    return 0;
+}
 template <typename T, int L, bool YPASS>
 static int spass_LA(hit3d_ctx *c, int axis, bool fwd, cx<T> *base, int64_t fs, int pitch, int nf)
 {
+    if constexpr (std::is_same<T, double>::value)
+        if (c->gate && fwd) return spass_gated_L<L, YPASS>(c, axis, base, fs, pitch, nf);
     if (c->ctile == 3) {
         IOPlain<T, T, T> io;
-        io.gate = c->gate;
-        io.src = base; io.dst = base; io.fs_src = fs; io.fs_dst = fs; io.ncol = c->nh;
+            io.src = base; io.dst = base; io.fs_src = fs; io.fs_dst = fs; io.ncol = c->nh;
         if (axis == 1) { io.sa_src = io.sa_dst = pitch; io.so_src = io.so_dst = (int64_t)c->n * pitch; }
         else { io.sa_src = io.sa_dst = (int64_t)c->n * pitch; io.so_src = io.so_dst = pitch; }
         int rows = c->n;
@@ -630,7 +645,9 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
         const int mode = pass == 0 ? PRE_COPY : PRE_SHIFT;
         MARK(0);
         if (!(zin && pass == 0)) {
-            c->zcmax = pass == 0 ? c->d_cmax : nullptr;  // the x pass below takes its maximum
+            // the x pass below takes its maximum
+            if (c->n > kClearMaxN && pass == 0) H3D_CHECK(cudaMemsetAsync(c->d_cmax, 0, sizeof(unsigned long long), c->st));
+            c->zcmax = pass == 0 ? c->d_cmax : nullptr;
             const int rc = zinv<T>(c, 3, mode, 0, c->U, c->fs64, Wf(0), wfs, wp);
             c->zcmax = nullptr;
             H3D_TRY(rc);

@@ -37,7 +37,6 @@ template <typename T, typename TI, typename TO> struct IOPlain {
     int64_t sa_src, so_src, sa_dst, so_dst;
     int ncol;
     int n = 0, kl = -1, ks = -1, ko = -1;
-    const double *gate = nullptr;  // the pass is skipped unless *gate < 0
     // runs of a batch: nfr > 0 fields per run, run r's fields start rs_src /
     // rs_dst elements after run r-1's; grid index z = r * nfr + f
     int nfr = 0;
@@ -55,7 +54,7 @@ template <typename T, typename TI, typename TO> struct IOPlain {
         return b;
     }
     H3D_D int outer(int y) const { return ko >= 0 ? kept_index(y, n, ko) : y; }
-    H3D_D bool begin() const { return gate == nullptr || *gate < 0.0; }
+    template <int L> H3D_D bool begin() const { return true; }
     H3D_D cx<T> load(int f, int o, int c, int p) const
     {
         if (c >= ncol || (kl >= 0 && !kept(p, n, kl))) return mk<T>(0, 0);
@@ -65,6 +64,13 @@ template <typename T, typename TI, typename TO> struct IOPlain {
     {
         if (c < ncol && (ks < 0 || kept(p, n, ks))) dst[f * fs_dst + p * sa_dst + o * so_dst + c] = to_cx<TO>(v);
     }
+};
+// one run's pass that is skipped unless *gate < 0 (its own type: the test cost every
+// strided pass of 512^3 0.002-0.003 ms)
+template <typename T> struct IOGated : IOPlain<T, T, T> {
+    const double *gate;
+    H3D_D IOGated at(int z, int &f) const { f = z; return *this; }
+    template <int L> H3D_D bool begin() const { return *gate < 0.0; }
 };
 
 // Spectral pre-operations applied while reading the FP64 state in the first
@@ -85,6 +91,7 @@ enum PreMode : int {
     PRE_GRAD_Z = 12,   // du_f/dz to field 3 f + 2 of dst          (IODeriv makes the others)
 };
 
+constexpr int kClearMaxN = 128;
 // MODE is a compile-time PreMode so that the plain copy carries no per-element
 // branching or wavenumber arithmetic
 template <typename T, typename TO, int MODE> struct IOSpec {
@@ -98,12 +105,14 @@ template <typename T, typename TO, int MODE> struct IOSpec {
     int kl = -1, ko = -1;  // 2/3-rule pruning of the kz loads and the ky rows
     int nfr = 0;           // runs of a batch, as IOPlain::at
     int64_t rs_src = 0, rs_dst = 0;
-    // cleared by one thread: the Courant maximum of the x pass to come (a memset
-    // of its own is one more launch of a small grid's seven)
+    // cleared by one thread up to kClearMaxN: the Courant maximum of the x pass to
+    // come (a memset of its own is one more launch of a small grid's seven; at 512^3
+    // the test alone took the z inverse from 0.522 to 0.546 ms)
     unsigned long long *zero = nullptr;
-    H3D_D bool begin() const
+    template <int L> H3D_D bool begin() const
     {
-        if (zero != nullptr && threadIdx.x == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) *zero = 0;
+        if constexpr (L <= kClearMaxN)
+            if (zero != nullptr && threadIdx.x == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) *zero = 0;
         return true;
     }
     H3D_D IOSpec at(int z, int &f) const
@@ -233,7 +242,7 @@ template <bool GRAD> struct IODeriv {
     int ncol, n, kl = -1;
     H3D_D IODeriv at(int z, int &f) const { f = z; return *this; }
     H3D_D int outer(int y) const { return y; }
-    H3D_D bool begin() const { return true; }
+    template <int L> H3D_D bool begin() const { return true; }
     H3D_D double2 load(int f, int o, int c, int p) const
     {
         if (c >= ncol || (kl >= 0 && !kept(p, n, kl))) return make_double2(0.0, 0.0);
@@ -274,7 +283,7 @@ __global__ void __launch_bounds__(NT, MINB) k_colfft(const IO io, const cx<T> *_
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T> *sm = reinterpret_cast<cx<T> *>(smraw);
     using F = ColFFT<T, L, TC, NT, false, FWD, false>;
-    if (!io.begin()) return;
+    if (!io.template begin<L>()) return;
     int f;
     const IO iob = io.at(blockIdx.z, f);
     const int col0 = blockIdx.x * TC, outer = iob.outer(blockIdx.y);
@@ -461,7 +470,7 @@ __global__ void __launch_bounds__(NT) k_xc2r_sums(const cx<TS> *base, int64_t fs
     }
 }
 
-// plain r2c (forward x pass) of one field, in place; gate (may be null) as IOPlain::gate
+// plain r2c (forward x pass) of one field, in place; gate (may be null) as IOGated::gate
 template <typename T, int L, int TC, int NT, typename TS>
 __global__ void __launch_bounds__(NT) k_xr2c(cx<TS> *base, int64_t fs, int64_t pitch, int npairs,
                                              const cx<T> *__restrict__ tw, int kx_lim, const double *gate)
