@@ -520,7 +520,7 @@ static int ensure_alias_state(hit3d_ctx *c)
         unsigned long long *d = reinterpret_cast<unsigned long long *>(c->d_red);
         H3D_CHECK(cudaMemsetAsync(d, 0, sizeof(unsigned long long), c->st));
         // a k_sgs beyond N/3 (brought there by clipping) keeps its own passes unpruned
-        k_alias_max<<<pw_grid(c), 256, 0, c->st>>>(c->n, c->nh, c->P64, c->fs64, 3 + c->nsc, c->U,
+        k_alias_any<<<pw_grid(c), 256, 0, c->st>>>(c->n, c->nh, c->P64, c->fs64, 3 + c->nsc, c->U,
                                                    3 + c->nsc - (c->p.les_model == 2 ? 1 : 0), c->RO, d);
         H3D_LAUNCH_CHECK();
         unsigned long long bits = 1;

@@ -550,27 +550,27 @@ __global__ void k_dealias_all(int n, int nh, int pitch, int64_t fs, int nf, int 
     }
 }
 
-// max |component| of nfa fields of A and nf of B over the modes the 2/3 rule
-// removes (some |k_i| > N/3), as the bit pattern of a non-negative double: zero
-// means the transforms of a time step may skip those modes exactly
-__global__ void k_alias_max(int n, int nh, int pitch, int64_t fs, int nf, const double2 *__restrict__ A, int nfa,
+// whether any component of nfa fields of A and nf of B is not zero at the modes the
+// 2/3 rule removes (some |k_i| > N/3): *out stays zero when the transforms of a
+// time step may skip those modes exactly.  The bits are looked at, without the
+// sign, so that a NaN counts (a floating-point maximum drops it).
+__global__ void k_alias_any(int n, int nh, int pitch, int64_t fs, int nf, const double2 *__restrict__ A, int nfa,
                             const double2 *__restrict__ B, unsigned long long *out)
 {
     const int64_t nm = (int64_t)n * n * nh;
     const ModeLoop ml(n, nh, -1);
-    double mx = 0.0;
+    unsigned long long any = 0;
+    auto bits = [](double2 v) {
+        return (unsigned long long)(__double_as_longlong(v.x) | __double_as_longlong(v.y)) << 1;
+    };
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nm; t += (int64_t)gridDim.x * blockDim.x) {
         const ModeIdx m = ml.at(t);
         if (m.ialias > 0) {
             const int64_t o = soff(m, n, pitch);
-            for (int f = 0; f < nf; f++) {
-                const double2 a = f < nfa ? A[o + f * fs] : make_double2(0.0, 0.0), b = B[o + f * fs];
-                mx = fmax(mx, fmax(fmax(fabs(a.x), fabs(a.y)), fmax(fabs(b.x), fabs(b.y))));
-            }
+            for (int f = 0; f < nf; f++) any |= (f < nfa ? bits(A[o + f * fs]) : 0ull) | bits(B[o + f * fs]);
         }
     }
-    for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    if ((threadIdx.x & 31) == 0 && mx > 0.0) atomicMax(out, (unsigned long long)__double_as_longlong(mx));
+    if (__any_sync(0xffffffffu, any != 0) && (threadIdx.x & 31) == 0) *out = 1;
 }
 
 // number of non-finite components among the N^2 (N/2+1) modes of nf fields of
