@@ -2199,6 +2199,7 @@ extern "C" int hit3d_gpu_init_velocity(hit3d_ctx *c, double rn1, int32_t isp, do
                 }
         H3D_TRY(upload_phys(c, g.data(), (int64_t)ld, 3));
         H3D_TRY(fwd3d64(c, c->W64, 3));
+        c->alias_known = 0;
         H3D_CHECK(cudaMemcpyAsync(c->U, c->W64, sizeof(double2) * 3 * c->fs64, cudaMemcpyDeviceToDevice, c->st));
         H3D_CHECK(cudaStreamSynchronize(c->st));
         return 0;
