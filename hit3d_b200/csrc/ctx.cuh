@@ -107,7 +107,7 @@ constexpr int kCopyStreams = 2;  // copy streams per direction of hit3d_gpu_step
 // replayed only while all of it is what it was at the recording
 struct StepKey {
     hit3d_params p;
-    int32_t es, int_scalars, idle_passive, xcfg, ctile, kc, pscheme, mlp_clip, mlp_kernel, pad;
+    int32_t es, int_scalars, idle_passive, xcfg, ctile, fuse_update, kc, pscheme, mlp_clip, mlp_kernel;
     int64_t np;
     double mlp_delta;
     const void *ptr[6];

@@ -1652,6 +1652,7 @@ static StepKey step_key(const hit3d_ctx *c, int es)
     k.idle_passive = c->idle_passive;
     k.xcfg = c->xcfg;
     k.ctile = c->ctile;
+    k.fuse_update = c->fuse_update;
     k.kc = (c->prune_on && c->pruned && c->p.dealias == 0) ? c->n / 3 : -1;
     k.pscheme = c->pscheme;
     k.mlp_clip = c->mlp_clip;
