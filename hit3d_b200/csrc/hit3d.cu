@@ -478,6 +478,12 @@ static int les_nles(int model)
     return (model == 2 || model == 4 || model == 6) ? 1 : (model == 3 || model == 5 || model == 7) ? 3
                                                                                                 : model == 10 ? 2 : 0;
 }
+// models whose pruned step is the unpruned one bit for bit.  A clipped k_sgs brings
+// modes beyond N/3 into the state: les_model 2 prunes everything else (128^3: 0.99
+// ms per step unpruned, 0.72 ms with all but k_sgs pruned).  The others with LES
+// fields prune nothing: k_sgs and its gradient of les_model 3, and the test filter
+// of 4-7 and 10, which takes products beyond N/3.
+static bool prune_exact(int model) { return les_nles(model) == 0 || model == 2; }
 static bool les_dlm(int model) { return model == 2 || model == 3; }
 static bool les_dstm(int model) { return model >= 4 && model <= 7; }
 // work fields of the Dynamic Structure models past the products (k_dstm_phys layout)
@@ -1093,10 +1099,7 @@ static int ctx_init(const hit3d_params *p, hit3d_ctx **out, double2 *ext_U, doub
     c->int_scalars = c->nsc > 0;
     c->xcfg = 4;  // register-resident fused x pass, the tuner's usual pick
     c->fuse_update = 0;  // the separate z pass + update measured faster so far
-    // a clipped k_sgs brings modes beyond N/3 into the state: les_model 2 prunes
-    // everything else, the other models with LES fields nothing (128^3, les_model 2:
-    // 0.99 ms per step unpruned, 0.72 ms with all but k_sgs pruned)
-    c->prune_on = les_nles(p->les_model) == 0 || p->les_model == 2;
+    c->prune_on = prune_exact(p->les_model);
     c->kc_active = -1;
     cudaDeviceProp prop;
     H3D_CHECK(cudaGetDeviceProperties(&prop, c->dev));
@@ -1960,7 +1963,7 @@ extern "C" int hit3d_gpu_set_update_fusion(hit3d_ctx *c, int32_t on)
 extern "C" int hit3d_gpu_set_pruning(hit3d_ctx *c, int32_t on)
 {
     if (!c) return h3d_set_error_msg(-1, "null context");
-    c->prune_on = on != 0;
+    c->prune_on = on != 0 && prune_exact(c->p.les_model);
     c->alias_known = 0;
     return 0;
 }

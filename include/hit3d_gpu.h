@@ -191,8 +191,9 @@ int hit3d_gpu_set_variant(hit3d_ctx *ctx, int32_t variant);
  * result is bit-identical; the state is checked on the device before the
  * first step after every change, and a state with energy beyond N/3 runs the
  * full transforms.  With les_model 2 everything but k_sgs is pruned (clipping
- * brings k_sgs modes beyond N/3).  hit3d_gpu_pruned returns 1 if the next step
- * is pruned. */
+ * brings k_sgs modes beyond N/3); les_models 3-7 and 10 are never pruned, the
+ * switch has no effect there (their clipped fields or filtered products hold
+ * modes beyond N/3).  hit3d_gpu_pruned returns 1 if the next step is pruned. */
 int hit3d_gpu_set_pruning(hit3d_ctx *ctx, int32_t on);
 int hit3d_gpu_pruned(hit3d_ctx *ctx);
 
