@@ -2680,8 +2680,7 @@ struct hit3d_batch {
     cudaGraphExec_t exec = nullptr;
     int graph_steps = 0;
     int64_t launches = 0;
-    std::vector<double> cap_dt;  // dt, scalar switch and pruning of every run when the graph was recorded
-    std::vector<int> cap_scal, cap_prune;
+    std::vector<StepKey> cap;  // what every run's launches depend on, when the graph was recorded
 };
 
 static int run_step(hit3d_ctx *c, int ev, int es)
@@ -3023,14 +3022,8 @@ static int batch_capture(hit3d_batch *b, int steps)
     b->graph = g;
     H3D_CHECK(cudaGraphInstantiate(&b->exec, g, 0));
     b->graph_steps = steps;
-    b->cap_dt.clear();
-    b->cap_scal.clear();
-    b->cap_prune.clear();
-    for (hit3d_ctx *cr : b->runs) {
-        b->cap_dt.push_back(cr->p.dt);
-        b->cap_scal.push_back(cr->int_scalars);
-        b->cap_prune.push_back(cr->prune_on && cr->pruned);
-    }
+    b->cap.clear();
+    for (hit3d_ctx *cr : b->runs) b->cap.push_back(step_key(cr, 0));
     return 0;
 }
 
@@ -3073,10 +3066,11 @@ extern "C" int hit3d_batch_step(hit3d_batch *b, int32_t nsteps, int32_t graph_st
         left--;
     }
     if (left >= graph_steps) {
-        bool stale = !b->exec || b->graph_steps != graph_steps || b->cap_dt.size() != b->runs.size();
-        for (size_t r = 0; !stale && r < b->runs.size(); r++)
-            stale = b->cap_dt[r] != b->runs[r]->p.dt || b->cap_scal[r] != b->runs[r]->int_scalars ||
-                    b->cap_prune[r] != (b->runs[r]->prune_on && b->runs[r]->pruned);
+        bool stale = !b->exec || b->graph_steps != graph_steps || b->cap.size() != b->runs.size();
+        for (size_t r = 0; !stale && r < b->runs.size(); r++) {
+            const StepKey k = step_key(b->runs[r], 0);
+            stale = memcmp(&k, &b->cap[r], sizeof k) != 0;
+        }
         if (stale) {
             for (hit3d_ctx *cr : b->runs) H3D_CHECK(cudaStreamSynchronize(cr->st));
             H3D_TRY(batch_capture(b, graph_steps));

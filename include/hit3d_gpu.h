@@ -342,10 +342,10 @@ int hit3d_gpu_physical_velocity(hit3d_ctx *ctx, double *out, int64_t ld1);
  * energy in device tables).  Other runs step on their own.  hit3d_batch_step
  * takes the first-order step of new runs eagerly, then records `graph_steps`
  * Adams-Bashforth steps of all classes and runs into one CUDA graph (a branch
- * per class or lone run) and replays it, one launch per chunk.  dt and the
- * scalar switch are baked into the recording: change them (hit3d_gpu_set_dt,
- * hit3d_gpu_set_scalars_active on a run's context) only between calls; the next
- * call re-records the graph when either, or graph_steps, has changed.
+ * per class or lone run) and replays it, one launch per chunk.  A run's dt,
+ * switches, launch shapes, particles and closure are baked into the recording:
+ * change them (on the run's context) only between calls; the next call
+ * re-records the graph when any of them, or graph_steps, has changed.
  * ------------------------------------------------------------------------- */
 typedef struct hit3d_batch hit3d_batch;
 int hit3d_batch_create(const hit3d_params *p /* [nruns] */, int32_t nruns, hit3d_batch **out);
