@@ -180,7 +180,8 @@ struct hit3d_ctx {
     StepKey sg_key;
     int64_t sg_kernels;
     int sg_seen;
-    unsigned long long *h_words;  // pinned: the Courant maximum and the error word of a call
+    unsigned long long *h_words;  // host: the Courant maximum and the error word of a call
+    int h_pinned;                 // h_words is page-locked
     int ext_bufs;        // U, RO and W belong to a batch's slab
     int ctile;           // column-tile shape of the plain strided passes (ColCfgT), grids up to 512
     // while a batch class is being stepped through this context (its first
