@@ -134,8 +134,7 @@ struct hit3d_ctx {
     const double *gate;  // set while passes are issued that run only if *gate < 0 on the device
     unsigned long long *zcmax;  // set while the z pass that clears the Courant maximum is issued
     int *d_err;          // device error word: bit 1 = a fused x pass gave up waiting for its input stage
-    double2 *stage;      // nstage fields in the reference layout: every state field up to 128^3, else one
-    int nstage;
+    double2 *stage;      // one field in the reference layout
     double *d_xyz, *d_uvw;
     int64_t np;
     int pscheme;

@@ -1155,7 +1155,6 @@ static int ctx_init(const hit3d_params *p, hit3d_ctx **out, double2 *ext_U, doub
     if (c->p.precision == 0) c->W64 = reinterpret_cast<double2 *>(c->W);
     else if ((rc = ctx_alloc((void **)&c->W64, f64 * 3))) { hit3d_gpu_finalize(c); return rc; }
     c->pblocks = c->nsm * 2;
-    c->nstage = c->n <= 128 ? 3 + c->nsc : 1;
     // per statistics block (two per SM): shells and the Parseval sum, or four sums of
     // up to kSumBlocks / 2 x-pass blocks
     const int kpart = c->kmax + 1 > 2 * kSumBlocks ? c->kmax + 1 : 2 * kSumBlocks;
@@ -1164,7 +1163,7 @@ static int ctx_init(const hit3d_params *p, hit3d_ctx **out, double2 *ext_U, doub
         (rc = ctx_alloc((void **)&c->d_part, sizeof(double) * (size_t)c->pblocks * kpart)) ||
         (rc = ctx_alloc((void **)&c->d_red, sizeof(double) * (size_t)(c->kmax + 1 + 12))) ||
         (rc = ctx_alloc((void **)&c->d_ratio, sizeof(double) * (size_t)kpart)) ||
-        (rc = ctx_alloc((void **)&c->stage, sizeof(double2) * (size_t)c->nstage * c->n * c->n * c->nh))) {
+        (rc = ctx_alloc((void **)&c->stage, sizeof(double2) * (size_t)c->n * c->n * c->nh))) {
         hit3d_gpu_finalize(c);
         return rc;
     }
@@ -1284,6 +1283,10 @@ extern "C" void hit3d_gpu_finalize(hit3d_ctx *c)
     delete c;
 }
 
+// largest grid whose transfers move all fields with one kernel and one copy; above
+// it a field's copy alone takes milliseconds and the launches do not count
+constexpr int kOneCopyMaxN = 128;
+
 static int transfer_fields(hit3d_ctx *c, double2 *dev, const double *hsrc, double *hdst, int64_t ld1, int nf)
 {
     if (!c) return h3d_set_error_msg(-1, "null context");
@@ -1294,19 +1297,23 @@ static int transfer_fields(hit3d_ctx *c, double2 *dev, const double *hsrc, doubl
     const size_t hp = (size_t)ld1 * sizeof(double);
     const size_t rows = (size_t)c->n * c->n;
     if (hsrc) c->alias_known = 0;
-    if (nf <= c->nstage && hp == width) {
+    if (c->n <= kOneCopyMaxN && hp == width) {
         // small grids: all fields with one kernel and one copy, a few microseconds
-        // each whatever the size (96 runs of 32^3 to 128^3 download 288 fields)
+        // each whatever the size (96 runs of 32^3 to 128^3 download 288 fields),
+        // through the work fields: at least 6 + 3 nsc of the transform precision,
+        // which hold 3 + nsc fields of the reference layout in either precision, and
+        // nothing lives there between calls
+        double2 *st = reinterpret_cast<double2 *>(c->W);
         const size_t bytes = width * rows * nf;
         const dim3 g((unsigned)std::min<int64_t>(pw_grid(c).x, ((int64_t)rows * c->nh + 255) / 256), nf);
         if (hsrc) {
-            H3D_CHECK(cudaMemcpyAsync(c->stage, hsrc, bytes, cudaMemcpyHostToDevice, c->st));
-            k_ref_to_dev<<<g, 256, 0, c->st>>>(c->n, c->nh, c->P64, c->stage, dev, c->fs64);
+            H3D_CHECK(cudaMemcpyAsync(st, hsrc, bytes, cudaMemcpyHostToDevice, c->st));
+            k_ref_to_dev<<<g, 256, 0, c->st>>>(c->n, c->nh, c->P64, st, dev, c->fs64);
             H3D_LAUNCH_CHECK();
         } else {
-            k_dev_to_ref<<<g, 256, 0, c->st>>>(c->n, c->nh, c->P64, dev, c->stage, c->fs64);
+            k_dev_to_ref<<<g, 256, 0, c->st>>>(c->n, c->nh, c->P64, dev, st, c->fs64);
             H3D_LAUNCH_CHECK();
-            H3D_CHECK(cudaMemcpyAsync(hdst, c->stage, bytes, cudaMemcpyDeviceToHost, c->st));
+            H3D_CHECK(cudaMemcpyAsync(hdst, st, bytes, cudaMemcpyDeviceToHost, c->st));
         }
         H3D_CHECK(cudaStreamSynchronize(c->st));
         return 0;
