@@ -113,6 +113,10 @@ struct StepKey {
     const void *ptr[6];
 };
 
+// step recordings (take_step in hit3d.cu): largest grid, the first wait, and the
+// replays that earn a recording's cost back
+constexpr int kGraphMaxN = 128, kGraphAfter = 8, kGraphEarn = 12;
+
 struct hit3d_ctx {
     hit3d_params p;
     int n, nh, P64, P32, nsc, dev, kmax, nsm;
@@ -173,12 +177,13 @@ struct hit3d_ctx {
     double2 *sin, *sout[2];  // one input staging set, two output sets used in turn
     int nstage_io;           // fields each staging set holds
     cudaEvent_t ev_in_ready, ev_in_free, ev_out_ready, ev_out_free[2];
-    // one Adams-Bashforth step recorded as a graph (grids up to 128), its key,
-    // its kernels, and the steps taken with the current key
+    // one Adams-Bashforth step recorded as a graph (grids up to 128), its key, its
+    // kernels and replays, the steps issued with the current key and how many of
+    // them a recording waits for; all recordings and replays so far
     cudaGraphExec_t sg;
     StepKey sg_key;
-    int64_t sg_kernels;
-    int sg_seen;
+    int64_t sg_kernels, sg_replays, sg_recorded, sg_replayed;
+    int sg_seen, sg_wait;
     unsigned long long *h_words;  // host: the Courant maximum and the error word of a call
     int h_pinned;                 // h_words is page-locked
     int ext_bufs;        // U, RO and W belong to a batch's slab

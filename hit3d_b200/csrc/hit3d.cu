@@ -1101,6 +1101,7 @@ static int ctx_init(const hit3d_params *p, hit3d_ctx **out, double2 *ext_U, doub
     c->fuse_update = 0;  // the separate z pass + update measured faster so far
     c->prune_on = prune_exact(p->les_model);
     c->kc_active = -1;
+    c->sg_wait = kGraphAfter;
     cudaDeviceProp prop;
     H3D_CHECK(cudaGetDeviceProperties(&prop, c->dev));
     c->nsm = prop.multiProcessorCount;
@@ -1659,15 +1660,18 @@ static bool chain_ok(const hit3d_ctx *c)
 }
 
 // A step of a grid up to 128 is 7 to 40 launches of a few microseconds each, and
-// issuing them takes the host longer than the GPU needs (64^3 decaying, 20 calls
-// of one step and a download: 1.33 ms issued one by one, 1.07 replayed; 128^3
-// Smagorinsky, 50 steps: 18.0 -> 16.9 ms).  After kGraphAfter Adams-Bashforth
-// steps with one key the step is recorded, and later steps with the same key
-// replay it with one launch; any change of the key drops the recording.  Below
-// kGraphAfter a run of a few steps would not earn back the recording (about ten
-// steps' saving); above 128 the kernels are long enough to hide their launches.
-constexpr int kGraphMaxN = 128, kGraphAfter = 4;
-
+// issuing them takes the host longer than the GPU needs (64^3 decaying: a one-step
+// call 63 us issued, 43 replayed, a step of a longer call 46 and 36; 128^3
+// Smagorinsky 343 and 322), so that an Adams-Bashforth step is recorded as a graph
+// and replayed with one launch.  A recording costs 70 to 110 us, what eight to
+// twelve replays save, and any change of the key (StepKey) drops it.  So it is made
+//   - inside a call whose remaining steps are sure to earn it back (kGraphEarn), after
+//     one step issued with the same key;
+//   - else once sg_wait steps have had the same key, while the GPU finishes the last
+//     step of a call.  sg_wait starts at kGraphAfter and doubles whenever a recording
+//     is dropped before it has earned its cost: with four steps' wait and no doubling,
+//     a dt that changed every six steps took 64^3 from 44.9 to 51.3 us a step.
+// Above 128 the kernels are long enough to hide their launches.
 static StepKey step_key(const hit3d_ctx *c, int es)
 {
     StepKey k;
@@ -1691,33 +1695,48 @@ static StepKey step_key(const hit3d_ctx *c, int es)
 }
 static void drop_step_graph(hit3d_ctx *c)
 {
-    if (c->sg) cudaGraphExecDestroy(c->sg);
+    if (c->sg) {
+        cudaGraphExecDestroy(c->sg);
+        c->sg_wait = c->sg_replays >= kGraphEarn ? kGraphAfter : c->sg_wait < (1 << 20) ? 2 * c->sg_wait : c->sg_wait;
+    }
     c->sg = nullptr;
     c->sg_seen = 0;
 }
 // record one Adams-Bashforth step; a recording that cannot be made leaves the
 // steps to be issued one by one (sg_seen far below zero)
-static int record_step(hit3d_ctx *c, int es)
+static void record_step(hit3d_ctx *c, int es)
 {
     const int64_t n0 = c->nlaunch;
-    H3D_CHECK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-    const int rc = c->p.precision == 0 ? step_once<double>(c, 0, es) : step_once<float>(c, 0, es);
     cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamEndCapture(c->st, &g);
-    if (rc == 0 && e == cudaSuccess) e = cudaGraphInstantiate(&c->sg, g, 0);
+    cudaError_t e = cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+        const int rc = c->p.precision == 0 ? step_once<double>(c, 0, es) : step_once<float>(c, 0, es);
+        e = cudaStreamEndCapture(c->st, &g);
+        if (rc != 0) e = cudaErrorStreamCaptureInvalidated;
+    }
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&c->sg, g, 0);
     if (g) cudaGraphDestroy(g);
     c->sg_kernels = c->nlaunch - n0;
     c->nlaunch = n0;
-    if (rc != 0 || e != cudaSuccess) {
+    c->sg_replays = 0;
+    if (e != cudaSuccess) {
         (void)cudaGetLastError();
         c->sg = nullptr;
         c->sg_seen = INT32_MIN / 2;
+        return;
     }
-    return 0;
+    c->sg_recorded++;
+}
+// at the end of a call, while the GPU works: the recording that is due
+static void record_if_due(hit3d_ctx *c)
+{
+    if (c->sg || c->sg_seen < c->sg_wait) return;
+    const StepKey k = step_key(c, c->sg_key.es);
+    if (memcmp(&k, &c->sg_key, sizeof k) == 0) record_step(c, c->sg_key.es);
 }
 // one step: euler_v, euler_s as step_once; Adams-Bashforth steps of small grids
-// through the recorded graph
-static int take_step(hit3d_ctx *c, int ev, int es, bool zin, bool zout)
+// through the recorded graph.  left: steps of the call from this one on
+static int take_step(hit3d_ctx *c, int ev, int es, bool zin, bool zout, int left)
 {
     if (c->n <= kGraphMaxN && !ev && !zin && !zout && c->bruns == 0) {
         const StepKey k = step_key(c, es);
@@ -1725,12 +1744,15 @@ static int take_step(hit3d_ctx *c, int ev, int es, bool zin, bool zout)
             drop_step_graph(c);
             c->sg_key = k;
         }
-        if (!c->sg && ++c->sg_seen > kGraphAfter) H3D_TRY(record_step(c, es));
+        if (!c->sg && c->sg_seen >= 1 && left >= kGraphEarn) record_step(c, es);
         if (c->sg) {
             H3D_CHECK(cudaGraphLaunch(c->sg, c->st));
             c->nlaunch += c->sg_kernels;
+            c->sg_replays++;
+            c->sg_replayed++;
             return 0;
         }
+        c->sg_seen++;
     }
     return c->p.precision == 0 ? step_once<double>(c, ev, es, nullptr, zin, zout)
                                : step_once<float>(c, ev, es, nullptr, zin, zout);
@@ -1748,7 +1770,7 @@ extern "C" int hit3d_gpu_step(hit3d_ctx *c, int32_t nsteps, int32_t *fov, int32_
     const bool chain = chain_ok(c);
     for (int it = 0; it < nsteps; it++) {
         const bool zin = chain && it > 0, zout = chain && it + 1 < nsteps;
-        H3D_TRY(take_step(c, ev, es, zin, zout));
+        H3D_TRY(take_step(c, ev, es, zin, zout, nsteps - it));
         ev = 0;
         if (c->int_scalars) es = 0;
     }
@@ -1764,6 +1786,7 @@ extern "C" int hit3d_gpu_step(hit3d_ctx *c, int32_t nsteps, int32_t *fov, int32_
         // the Courant maximum and the error word in one read
         unsigned long long *words = c->h_words;
         H3D_CHECK(cudaMemcpyAsync(words, c->d_cmax, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->st));
+        record_if_due(c);
         H3D_CHECK(cudaStreamSynchronize(c->st));
         int derr = 0;
         memcpy(&derr, &words[1], sizeof derr);
@@ -1802,6 +1825,13 @@ extern "C" int hit3d_gpu_les_set_mlp(hit3d_ctx *c, const uint16_t *wb, int64_t n
 
 extern "C" void *hit3d_gpu_stream(hit3d_ctx *c) { return c ? (void *)c->st : nullptr; }
 extern "C" int64_t hit3d_gpu_launch_count(hit3d_ctx *c) { return c ? c->nlaunch : -1; }
+extern "C" int hit3d_gpu_step_graph(hit3d_ctx *c, int64_t *recorded, int64_t *replayed)
+{
+    if (!c || !recorded || !replayed) return h3d_set_error_msg(-1, "hit3d_gpu_step_graph: null argument");
+    *recorded = c->sg_recorded;
+    *replayed = c->sg_replayed;
+    return 0;
+}
 
 extern "C" int hit3d_gpu_step_profile(hit3d_ctx *c, int32_t nsteps, int32_t *fov, int32_t *fos, double *ms)
 {

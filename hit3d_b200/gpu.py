@@ -117,6 +117,7 @@ SIGNATURES = [
     ("hit3d_gpu_restart_unpack", C.c_int, [_vp, C.c_void_p, _i64, _dp, _dp, C.POINTER(_i32), C.POINTER(_i32)]),
     ("hit3d_gpu_stream", C.c_void_p, [_vp]),
     ("hit3d_gpu_launch_count", C.c_int64, [_vp]),
+    ("hit3d_gpu_step_graph", C.c_int, [_vp, C.POINTER(_i64), C.POINTER(_i64)]),
     ("hit3d_gpu_autotune", C.c_int, [_vp, C.POINTER(_i32), _dp]),
     ("hit3d_gpu_autotune_columns", C.c_int, [_vp, C.POINTER(_i32), _dp]),
     ("hit3d_gpu_set_column_tile", C.c_int, [_vp, _i32]),
@@ -383,6 +384,13 @@ class Context:
     def launches(self) -> int:
         """Kernels launched by this context so far."""
         return int(lib().hit3d_gpu_launch_count(self._h))
+
+    @property
+    def step_graph(self) -> tuple:
+        """(recordings, replayed steps) of this context's steps so far (grids up to 128)."""
+        r, q = C.c_int64(0), C.c_int64(0)
+        _check(lib().hit3d_gpu_step_graph(self._h, C.byref(r), C.byref(q)), "step_graph")
+        return r.value, q.value
 
     @property
     def stream(self) -> int:

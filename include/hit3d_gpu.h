@@ -224,6 +224,10 @@ int hit3d_gpu_les_stats(hit3d_ctx *ctx, double *out4);
 
 /* Number of kernels this context has launched since hit3d_gpu_init. */
 int64_t hit3d_gpu_launch_count(hit3d_ctx *ctx);
+/* Steps of a grid up to 128 that keep dt, switches, launch shapes and particles
+ * are replayed from a recorded graph, with the same results: how many recordings
+ * hit3d_gpu_step has made and how many steps it has replayed so far. */
+int hit3d_gpu_step_graph(hit3d_ctx *ctx, int64_t *recorded, int64_t *replayed);
 
 /* Change dt (my_dt.f90) and start/stop advancing scalars (int_scalars, main.f90:199-204). */
 int hit3d_gpu_set_dt(hit3d_ctx *ctx, double dt);
