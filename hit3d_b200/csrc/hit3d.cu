@@ -134,22 +134,25 @@ static int zinv_L(hit3d_ctx *c, int nf, int mode, int sfield, const double2 *src
     switch (mode) {
     case PRE_COPY: return zinv_LM<T, L, PRE_COPY>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
     case PRE_SHIFT: return zinv_LM<T, L, PRE_SHIFT>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
-    case PRE_STRAIN_A: return zinv_LM<T, L, PRE_STRAIN_A>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
-    case PRE_STRAIN_B: return zinv_LM<T, L, PRE_STRAIN_B>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
     case PRE_GRAD: return zinv_LM<T, L, PRE_GRAD>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
     case PRE_QUART: return zinv_LM<T, L, PRE_QUART>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
     default: break;
     }
     if constexpr (std::is_same<T, double>::value) {
-        // statistics pre-operations run in FP64 only
+        // statistics, the closures' z derivatives and the filters run in FP64 only
         switch (mode) {
         case PRE_STRAIN_Z: return zinv_LM<T, L, PRE_STRAIN_Z>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
         case PRE_GRAD_Z: return zinv_LM<T, L, PRE_GRAD_Z>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
-        case PRE_CURL: return zinv_LM<T, L, PRE_CURL>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
         case PRE_DLONG: return zinv_LM<T, L, PRE_DLONG>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
         case PRE_TRUNC: return zinv_LM<T, L, PRE_TRUNC>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
         case PRE_CUBE: return zinv_LM<T, L, PRE_CUBE>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
         case PRE_FILT: return zinv_LM<T, L, PRE_FILT>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
+        default: break;
+        }
+    } else {
+        switch (mode) {
+        case PRE_STRAIN_A: return zinv_LM<T, L, PRE_STRAIN_A>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
+        case PRE_STRAIN_B: return zinv_LM<T, L, PRE_STRAIN_B>(c, nf, sfield, src, src_fs, dst, dst_fs, dpitch);
         default: break;
         }
     }
@@ -253,7 +256,7 @@ static int spass_LA(hit3d_ctx *c, int axis, bool fwd, cx<T> *base, int64_t fs, i
         if (c->gate && fwd) return spass_gated_L<L, YPASS>(c, axis, base, fs, pitch, nf);
     if (c->ctile == 3) {
         IOPlain<T, T, T> io;
-            io.src = base; io.dst = base; io.fs_src = fs; io.fs_dst = fs; io.ncol = c->nh;
+        io.src = base; io.dst = base; io.fs_src = fs; io.fs_dst = fs; io.ncol = c->nh;
         if (axis == 1) { io.sa_src = io.sa_dst = pitch; io.so_src = io.so_dst = (int64_t)c->n * pitch; }
         else { io.sa_src = io.sa_dst = (int64_t)c->n * pitch; io.so_src = io.so_dst = pitch; }
         int rows = c->n;
@@ -582,8 +585,8 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
     const int nps = p.n_scalars, kf0 = 3 + p.n_scalars;  // kf0: first LES field of the state
     const int kf = nprod + (lag ? 18 : 10) + 3 * nps, nutf = kf + 1;
 
-    // FP64: the velocity's derivatives are made beside its own inverse (deriv_inv)
-    const bool deriv = std::is_same<T, double>::value && (les || les_mlp || dlm);
+    // FP64: the closures' velocity derivatives are made beside its own inverse (deriv_inv)
+    constexpr bool deriv = std::is_same<T, double>::value;
 
     MARK(7);
     if constexpr (std::is_same<T, double>::value) {
@@ -669,10 +672,10 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
         };
         for (int s = 0; s < ns; s++)
             H3D_TRY(field_pass(s, [&] { return zinv<T>(c, 1, mode, 0, c->U + (3 + s) * c->fs64, c->fs64, Wf(6 + 3 * s), wfs, wp); }));
-        if constexpr (std::is_same<T, double>::value) {
+        if constexpr (deriv) {
             // while the velocity's z inverse is there: strains or gradients of the
             // closures below, as far as their x pass
-            if (deriv) {
+            if (les || les_mlp || dlm) {
                 MARK(6);
                 if (les_mlp) H3D_TRY(deriv_inv<true>(c, Wf(0), Wf(nprod), wfs, wp));
                 else H3D_TRY(deriv_inv<false>(c, Wf(0), Wf(nprod), wfs, wp));
@@ -764,7 +767,7 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
             // fluxes nu_t grad(phi) from the physical fields (m_les.f90:1142-1215,
             // 902-1018, 1028-1091)
             const int t0 = nprod, nf = 6 + 3 * ns, y0 = deriv ? 6 : 0;
-            if (!deriv) {
+            if constexpr (!deriv) {
                 H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_A, 0, c->U, c->fs64, Wf(t0), wfs, wp));
                 H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_B, 0, c->U, c->fs64, Wf(t0 + 3), wfs, wp));
             }
@@ -785,7 +788,7 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
             MARK(6);
             // Smagorinsky stress from the same state (m_les.f90:1142-1215, 902-1018)
             const int t0 = nprod;
-            if (!deriv) {
+            if constexpr (!deriv) {
                 H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_A, 0, c->U, c->fs64, Wf(t0), wfs, wp));
                 H3D_TRY(zinv<T>(c, 3, PRE_STRAIN_B, 0, c->U, c->fs64, Wf(t0 + 3), wfs, wp));
                 H3D_TRY(spass<T>(c, 1, false, Wf(t0), wfs, wp, 6));
@@ -950,7 +953,7 @@ static int step_once(hit3d_ctx *c, int euler_v, int euler_s, Prof *prof = nullpt
             // learned closure: the nine velocity gradients in physical space, the
             // network per point, the six stresses back to spectral space
             const int t0 = nprod;
-            if (!deriv) {
+            if constexpr (!deriv) {
                 for (int i = 0; i < 3; i++) H3D_TRY(zinv<T>(c, 3, PRE_GRAD, i, c->U, c->fs64, Wf(t0 + 3 * i), wfs, wp));
                 H3D_TRY(spass<T>(c, 1, false, Wf(t0), wfs, wp, 9));
             }

@@ -78,10 +78,9 @@ template <typename T> struct IOGated : IOPlain<T, T, T> {
 enum PreMode : int {
     PRE_COPY = 0,      // field f of the state
     PRE_SHIFT = 1,     // field f times exp(i (kx+ky+kz) dx/2)   (rhs_velocity.f90:248-257)
-    PRE_CURL = 2,      // vorticity component f                 (m_stats.f90:260-274)
     PRE_DLONG = 3,     // du_f/dx_f                              (new: skewness)
-    PRE_STRAIN_A = 4,  // S11, S12, S13 for f = 0,1,2            (m_les.f90:1153-1170)
-    PRE_STRAIN_B = 5,  // S22, S23, S33 for f = 0,1,2            (m_les.f90:1180-1198)
+    PRE_STRAIN_A = 4,  // S11, S12, S13 for f = 0,1,2, FP32      (m_les.f90:1153-1170)
+    PRE_STRAIN_B = 5,  // S22, S23, S33 for f = 0,1,2, FP32      (m_les.f90:1180-1198)
     PRE_GRAD = 6,      // d phi/dx_f of state field `sfield`     (m_stats.f90:323-326)
     PRE_TRUNC = 7,     // field f with |k|^2 > k2max zeroed       (io_write_4.f90:21-42)
     PRE_CUBE = 8,      // field f with some |k_i| > N/3 zeroed    (m_les.f90:1579-1586)
@@ -91,6 +90,8 @@ enum PreMode : int {
     PRE_GRAD_Z = 12,   // du_f/dz to field 3 f + 2 of dst          (IODeriv makes the others)
 };
 
+// largest grid whose velocity z inverse clears the Courant maximum (IOSpec::begin);
+// above it the step issues a memset before that pass
 constexpr int kClearMaxN = 128;
 // MODE is a compile-time PreMode so that the plain copy carries no per-element
 // branching or wavenumber arithmetic
@@ -141,14 +142,6 @@ template <typename T, typename TO, int MODE> struct IOSpec {
             double2 u = U(f, o, c, p);
             const double2 w = __ldg(sh + (c + kwave(o, n) + kwave(p, n)));
             r = make_double2(u.x * w.x - u.y * w.y, u.y * w.x + u.x * w.y);
-            break;
-        }
-        case PRE_CURL: {
-            // x_derivative: (a + ib) k -> (-k b, k a); omega as the reference forms it
-            double2 u = U(0, o, c, p), v = U(1, o, c, p), w = U(2, o, c, p);
-            if (f == 0) r = make_double2((-(ky * w.y)) - (-(kz * v.y)), (ky * w.x) - (kz * v.x));       // w_y - v_z
-            else if (f == 1) r = make_double2((-(kz * u.y)) - (-(kx * w.y)), (kz * u.x) - (kx * w.x));  // u_z - w_x
-            else r = make_double2((-(kx * v.y)) - (-(ky * u.y)), (kx * v.x) - (ky * u.x));              // v_x - u_y
             break;
         }
         case PRE_DLONG: {
