@@ -2080,7 +2080,6 @@ extern "C" int hit3d_gpu_dealias_all(hit3d_ctx *c)
     return 0;
 }
 
-// shell spectrum of nf state fields starting at src -> host es[0..kmax)
 // device sums of the statistics, in d_red: shells 0..kmax-1, the Parseval sum at
 // kmax (m != SPEC_ONLY), the physical sums (four per field) from kmax + 1
 static int shell_sums(hit3d_ctx *c, const double2 *src, int nf, double w0, SpecMode m, int kc)
@@ -2101,6 +2100,7 @@ static int shell_sums(hit3d_ctx *c, const double2 *src, int nf, double w0, SpecM
     H3D_LAUNCH_CHECK();
     return 0;
 }
+// shell spectrum of nf fields starting at src -> host es[0..kmax)
 static int shell_spectrum(hit3d_ctx *c, const double2 *src, int nf, double *es, double w0 = 0.5)
 {
     H3D_TRY(shell_sums(c, src, nf, w0, SPEC_ONLY, -1));

@@ -350,7 +350,7 @@ static __global__ void __launch_bounds__(256, 2) k_mlp_grad(const MlpBatch b, co
             float *o = &v.x;
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                // gelu and gelu_d with one tanh
+                // gelu and its derivative with one tanh
                 const float zz = z[r][e], u = GELU_A * (zz + GELU_B * (zz * zz * zz)), t = tanhf(u);
                 o[e] = 0.5f * zz * (1.0f + t);
                 d[r][e] = 0.5f * (1.0f + t) + 0.5f * zz * (1.0f - t * t) * GELU_A * (1.0f + 3.0f * GELU_B * (zz * zz));

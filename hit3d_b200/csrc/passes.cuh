@@ -224,9 +224,9 @@ template <typename T, typename TO, int MODE> struct IOSpec {
 // z derivatives (in d, from PRE_STRAIN_Z / PRE_GRAD_Z) have z passes of their own:
 // three fields instead of six strains or nine gradients.
 //   GRAD: d = du_i/dx_j at 3 i + j; else d = S11, S12, S13, S22, S23, S33
-// Three z transforms and a launch or two less; what is left of these passes is
-// bound by shared-memory traffic (L1 75-89 %, DRAM below 41 % at 128^3).  128^3
-// FP64, per step: learned closure 0.598 -> 0.574 ms, Smagorinsky 0.328 -> 0.321.
+// Three z transforms and a launch or two less.  The y pass, pruned, at 128^3: 28 us
+// for six strains, 44 for nine gradients, L1 at 60-68 % and DRAM at 24-28 % of their
+// rates, the warps waiting for loads and the stages' barriers.  128^3 FP64, per step: learned closure 0.598 -> 0.574 ms, Smagorinsky 0.328 -> 0.321.
 // FP64 only: in the FP32 form ik before or after the z transform rounds apart.
 template <bool GRAD> struct IODeriv {
     const double2 *w;

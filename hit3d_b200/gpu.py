@@ -365,11 +365,12 @@ class Context:
         return dict(zip(("energy", "production", "B", "dissipation"), out.tolist()))
 
     def set_update_fusion(self, on: bool):
-        """Fuse the velocity products' z pass with the update (the default) or not."""
+        """Fuse the velocity products' z pass with the update, or not (the default)."""
         _check(lib().hit3d_gpu_set_update_fusion(self._h, int(bool(on))), "set_update_fusion")
 
     def set_pruning(self, on: bool):
-        """Allow (default) or forbid 2/3-rule pruning of the step's transforms."""
+        """Allow (default) or forbid 2/3-rule pruning of the step's transforms; no effect with
+        les_models 3-7 and 10, which are never pruned."""
         _check(lib().hit3d_gpu_set_pruning(self._h, int(bool(on))), "set_pruning")
 
     @property
