@@ -553,7 +553,7 @@ __global__ void k_dealias_all(int n, int nh, int pitch, int64_t fs, int nf, int 
 // whether any component of nfa fields of A and nf of B is not zero at the modes the
 // 2/3 rule removes (some |k_i| > N/3): *out stays zero when the transforms of a
 // time step may skip those modes exactly.  The bits are looked at, without the
-// sign, so that a NaN counts (a floating-point maximum drops it).
+// sign, so that a NaN counts (a floating-point maximum drops it).  3 <= nfa <= nf.
 __global__ void k_alias_any(int n, int nh, int pitch, int64_t fs, int nf, const double2 *__restrict__ A, int nfa,
                             const double2 *__restrict__ B, unsigned long long *out)
 {
@@ -567,7 +567,12 @@ __global__ void k_alias_any(int n, int nh, int pitch, int64_t fs, int nf, const 
         const ModeIdx m = ml.at(t);
         if (m.ialias > 0) {
             const int64_t o = soff(m, n, pitch);
-            for (int f = 0; f < nf; f++) any |= (f < nfa ? bits(A[o + f * fs]) : 0ull) | bits(B[o + f * fs]);
+            // the velocity's six loads together, then a pair at a time
+#pragma unroll
+            for (int f = 0; f < 3; f++) any |= bits(A[o + f * fs]) | bits(B[o + f * fs]);
+#pragma unroll 2
+            for (int f = 3; f < nfa; f++) any |= bits(A[o + f * fs]) | bits(B[o + f * fs]);
+            for (int f = nfa; f < nf; f++) any |= bits(B[o + f * fs]);
         }
     }
     if (__any_sync(0xffffffffu, any != 0) && (threadIdx.x & 31) == 0) *out = 1;
