@@ -193,7 +193,10 @@ int hit3d_gpu_set_variant(hit3d_ctx *ctx, int32_t variant);
  * full transforms.  With les_model 2 everything but k_sgs is pruned (clipping
  * brings k_sgs modes beyond N/3); les_models 3-7 and 10 are never pruned, the
  * switch has no effect there (their clipped fields or filtered products hold
- * modes beyond N/3).  hit3d_gpu_pruned returns 1 if the next step is pruned. */
+ * modes beyond N/3).  hit3d_gpu_pruned returns 1 if the next step is pruned.
+ * With a velocity beyond N/3 (an upload that was not dealiased) the k_sgs
+ * production of les_models 2, 3 and 5-7 takes the strain of every mode, where the
+ * reference truncates it (m_les.f90:1422-1561). */
 int hit3d_gpu_set_pruning(hit3d_ctx *ctx, int32_t on);
 int hit3d_gpu_pruned(hit3d_ctx *ctx);
 
